@@ -60,7 +60,7 @@ HL_API const char* hl_version(void);
  *   "d3q27_kernel": 0 automatic, 1 the asynchronous-copy kernel, 2 the TMA-staged kernel
  *   "d3q27_chunks": 0 automatic, k > 0 splits x into k chunks per tile column (read by
  *     hl_d3q27_stream_collide at launch and by hl_d3q27_batch_prepare)
- *   "d3q27_stages": 0 automatic (4), 3..5 planes staged by the TMA kernel
+ *   "d3q27_stages": 0, 3..5: accepted, without effect (the staging depth is fixed per storage type)
  *   "d3q27_link_blocks": 0 automatic, k > 0 blocks of the cut-link kernel over the listed
  *     cells (fewer leave SMs free for other domains' kernels on other streams): blocks of 16
  *     warps for hl_d3q27_solid_links (automatic: one per SM), of 4 warps for
@@ -150,7 +150,7 @@ HL_API size_t hl_d3q27_scratch_bytes(const hl_world3d* w);
  *    non-finite moments or rho <= 0); mass and health may be NULL. Storage float32 or
  *    float64 (other storages return HL_ERR_ARG); it always runs the general kernel, never
  *    the TMA-staged one, so its results can differ from hl_d3q27_stream_collide in rounding.
- *  - Limit: 16 + 12 bytes per CTA of scratch, i.e. devices with up to 1364 SMs (a B200 has
+ *  - Limit: 64 + 12 bytes for each of two CTAs per SM, i.e. devices with up to 680 SMs (a B200 has
  *    148); larger needs are rejected with HL_ERR_ARG.
  *  - The first call on a device resolves the array's device address (cudaGetSymbolAddress,
  *    with that device current); make that first call before any stream capture.

@@ -1,4 +1,9 @@
-// D3Q27 HOME-LBM step for sm_100a: stream-collide, outer boundaries, initial states.
+// D3Q27 stream-collide in binary32 for rows of any length, and the entry points of the step. Domains
+// whose rows are multiples of 16 bytes, binary64 and the 16-bit storages run the sweeps of
+// d3q27_sweep.cuh (d3q27_tma.cu; binary64 with other rows from here). For binary32 rows that
+// tensor copies cannot take, the sweeps staged by 4-byte asynchronous copies are the slower form
+// (200 x 150 x 133: 188 us a step against 164 us here; 60 x 47 x 53: 15.4 against 11.3): a warp of 16
+// column pairs stores such rows in parts of sectors, and this kernel's warps store whole rows.
 //
 // Stream-collide (replaces stream_and_collide_3d, envs/lbm3d/lbm_func_3d.py:364-604).
 // The reference pulls, for every cell and direction i, the population rebuilt from the
@@ -32,8 +37,9 @@
 
 #include <cstdio>
 #include <cstdlib>
+#include <cstring>
 
-#include "d3q27_core.cuh"
+#include "d3q27_sweep.cuh"
 
 namespace hl {
 namespace d3 {
@@ -261,13 +267,14 @@ template <int TY> Plan make_plan(int nx, int ny, int nz) {
   return p;
 }
 
-size_t diag_scratch_bytes() { return size_t(num_sms()) * (sizeof(double) + sizeof(int)) + 64; }
+// one partial sum and one count per block, after the completion counter
+size_t diag_scratch_bytes() { return size_t(sw::BLOCKS_PER_SM) * num_sms() * (sizeof(double) + sizeof(int)) + 64; }
 
 void fill_diag(StepArgs& a, const hl_diag* diag) {
   char* s = static_cast<char*>(diag->scratch);
   a.counter = reinterpret_cast<unsigned*>(s);
   a.partials = reinterpret_cast<double*>(s + 16);
-  a.bad_partials = reinterpret_cast<int*>(s + 16 + sizeof(double) * num_sms());
+  a.bad_partials = reinterpret_cast<int*>(s + 16 + sizeof(double) * sw::BLOCKS_PER_SM * num_sms());
   a.mass = diag->mass;
   a.health = diag->health;
 }
@@ -324,6 +331,13 @@ int dispatch_step(const hl_world3d* w, double vis, const hl_diag* d, cudaStream_
   return HL_ERR_UNSUPPORTED;
 }
 
+// binary64 with rows that are no multiple of 16 bytes: the sweeps staged by 8-byte copies
+int launch_sweep_f64(const hl_world3d* w, double vis, const hl_diag* diag, cudaStream_t st) {
+  sw::Maps unused;
+  std::memset(&unused, 0, sizeof(unused));
+  return sw::dispatch<StoreF64, false>(w, vis, diag, unused, st);
+}
+
 }  // namespace d3
 }  // namespace hl
 
@@ -343,10 +357,12 @@ extern "C" int hl_d3q27_stream_collide(const hl_world3d* w, double vis_shear, co
     set_error("d3q27: the TMA kernel needs ny %% 16 == 0, nz %% 32 == 0 and a non-float64 storage");
     return HL_ERR_UNSUPPORTED;
   }
-  if (g_tune_d3_kernel != 1 && d3::tma_eligible(w)) return d3::launch_step_tma(w, vis_shear, diag, st);
+  const bool plain = w->storage.dtype == HL_F32 || w->storage.dtype == HL_F64;
+  if (g_tune_d3_kernel != 1 && (plain ? d3::box_eligible(w) : d3::tma_eligible(w)))
+    return d3::launch_step_tma(w, vis_shear, diag, st);
   switch (w->storage.dtype) {
     case HL_F32: return d3::dispatch_step<16, StoreF32>(w, vis_shear, diag, st);
-    case HL_F64: return d3::dispatch_step<8, StoreF64>(w, vis_shear, diag, st);
+    case HL_F64: return d3::launch_sweep_f64(w, vis_shear, diag, st);
     default:
       set_error("d3q27: storage dtype %d not supported by this build", int(w->storage.dtype));
       return HL_ERR_UNSUPPORTED;
@@ -365,7 +381,7 @@ extern "C" size_t hl_d3q27_scratch_bytes(const hl_world3d*) { return d3::diag_sc
 namespace hl {
 namespace d3 {
 
-constexpr size_t kNoAllocScratchBytes = 16384;  // 16 + 12 bytes per CTA: up to 1364 CTAs (one per SM)
+constexpr size_t kNoAllocScratchBytes = 16384;  // 64 + 12 bytes per CTA, two CTAs per SM: up to 680 SMs
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratchBytes];
 
 // Device address of g_noalloc_scratch on the current device. The host-side symbol is only a
@@ -405,10 +421,8 @@ extern "C" int hl_d3q27_stream_collide_noalloc(const hl_world3d* w, double vis_s
   HL_CHECK_ARG(vis_shear > 0.0, "d3q27 (no-alloc): viscosity must be positive");
   HL_CHECK_ARG(w->storage.dtype == HL_F32 || w->storage.dtype == HL_F64,
                "d3q27 (no-alloc): storage must be float32 or float64");
-  const d3::Plan plan =
-      w->storage.dtype == HL_F32 ? d3::make_plan<16>(w->nx, w->ny, w->nz) : d3::make_plan<8>(w->nx, w->ny, w->nz);
-  const size_t need = 16 + size_t(d3::num_sms()) * (sizeof(double) + sizeof(int));
-  HL_CHECK_ARG(need <= d3::kNoAllocScratchBytes && size_t(plan.grid) <= size_t(d3::num_sms()),
+  const size_t need = d3::diag_scratch_bytes();
+  HL_CHECK_ARG(need <= d3::kNoAllocScratchBytes,
                "d3q27 (no-alloc): needs %zu bytes of scratch for %d SMs; the static scratch holds %zu", need,
                d3::num_sms(), d3::kNoAllocScratchBytes);
   void* scratch = nullptr;
@@ -421,5 +435,5 @@ extern "C" int hl_d3q27_stream_collide_noalloc(const hl_world3d* w, double vis_s
   if (e != cudaSuccess) return cuda_status(e, "hl_d3q27_stream_collide_noalloc: clear counter");
   hl_diag d{scratch, d3::kNoAllocScratchBytes, mass, health};
   return w->storage.dtype == HL_F32 ? d3::dispatch_step<16, StoreF32>(w, vis_shear, &d, st)
-                                    : d3::dispatch_step<8, StoreF64>(w, vis_shear, &d, st);
+                                    : d3::launch_sweep_f64(w, vis_shear, &d, st);
 }

@@ -9,6 +9,8 @@ namespace d3 {
 struct StepArgs {
   const void* cur;
   void* post;
+  const void* cur_k[10];  // cur's and post's ten moment planes
+  void* post_k[10];
   long long N;  // cells per field plane
   int nx, ny, nz;
   int tiles_y, tiles_z, n_tiles;
@@ -29,8 +31,11 @@ struct StepArgs {
 int num_sms();
 size_t diag_scratch_bytes();
 void fill_diag(StepArgs& a, const hl_diag* diag);
-// TMA-staged variant (d3q27_tma.cu): every tile full (ny % 16 == 0, nz % 32 == 0)
+// TMA-staged variant (d3q27_tma.cu): tma_eligible is what "d3q27_kernel" 2, the 16-bit storages and
+// the batched launch take (every tile full: ny % 16 == 0, nz % 32 == 0); box_eligible what the
+// automatic choice sends there in binary32 and binary64.
 bool tma_eligible(const hl_world3d* w);
+bool box_eligible(const hl_world3d* w);
 int launch_step_tma(const hl_world3d* w, double vis_shear, const hl_diag* diag, cudaStream_t st);
 
 // Partial moments of one destination cell.

@@ -763,21 +763,26 @@ template <class R> __device__ Mom2<R> bc_core(const World& w, int dr, const Mom2
   return r;
 }
 
-// One CTA per world. Threads of the reference run in launch order (x outer, y inner): a
-// corner reads a neighbour on a low face (x = 0 or y = 0) before that neighbour's update
-// and one on a high face after it. Phase 1 updates the non-corner border cells, saving the
-// four cells corners read "before update"; phase 2 updates the corners.
-template <class S> __global__ void __launch_bounds__(512) boundary_kernel(const __grid_constant__ Launch L) {
+// BC_BLOCKS blocks per world (blockIdx.x the world). Threads of the reference run in launch order (x outer, y
+// inner): a corner reads a neighbour on a low face (x = 0 or y = 0) before that neighbour's update and
+// one on a high face after it. Border cells read only the row inside them, so any block may take
+// any of them; the first warp of a world's first block takes the eight cells next to the corners,
+// keeping their old values, and then the corners. A cell is a chain of dependent loads, so the
+// threads in flight set the time: one 512-thread block a world took 18 us at 512 x 128 and 36 us for
+// 60 uneven worlds.
+constexpr int BC_BLOCKS = 12, BC_THREADS = 128;
+template <class S> __global__ void __launch_bounds__(BC_THREADS) boundary_kernel(const __grid_constant__ Launch L) {
   using R = typename S::R;
   using T = typename S::T;
   const World& w = world_of(L, blockIdx.x);
+  const int part = blockIdx.y;
   const long long N = (long long)w.nx * w.ny;
   T* post = static_cast<T*>(post_of(L, w));
-  __shared__ R snap[4][7];  // (1,0) (0,1) (1,ny-1) (nx-1,1)
+  const int tid = threadIdx.x;
   if (!w.periodic) {
     const int ex = w.nx - 2, ey = w.ny - 2;  // border cells per side without corners
-    const int total = 2 * ey + 2 * ex;
-    for (int k = threadIdx.x; k < total; k += blockDim.x) {
+    // border cell k of the four sides in turn and the cell inside it
+    auto update = [&](int k, Mom2<R>* old) {
       int x, y, dr, xn, yn;
       if (k < ey) { x = 0; y = 1 + k; dr = 0; xn = 1; yn = y; }
       else if (k < 2 * ey) { x = w.nx - 1; y = 1 + k - ey; dr = 2; xn = w.nx - 2; yn = y; }
@@ -785,42 +790,45 @@ template <class S> __global__ void __launch_bounds__(512) boundary_kernel(const 
       else { x = 1 + k - 2 * ey - ex; y = 0; dr = 3; xn = x; yn = 1; }
       const long long c = (long long)x * w.ny + y;
       const Mom2<R> t = load2<S>(w, N, c, post);
-      int slot = -1;
-      if (x == 1 && y == 0) slot = 0;
-      else if (x == 0 && y == 1) slot = 1;
-      else if (x == 1 && y == w.ny - 1) slot = 2;
-      else if (x == w.nx - 1 && y == 1) slot = 3;
-      if (slot >= 0) {
-        snap[slot][0] = t.rho; snap[slot][1] = t.ux; snap[slot][2] = t.uy;
-        snap[slot][3] = t.sxx; snap[slot][4] = t.syy; snap[slot][5] = t.sxy; snap[slot][6] = t.drho;
-      }
+      if (old) *old = t;
       store2<S>(w, N, c, post, bc_core<R>(w, dr, t, load2<S>(w, N, (long long)xn * w.ny + yn, post)));
-    }
-    __syncthreads();
-    if (threadIdx.x < 4) {
-      const int k = threadIdx.x;
-      const int x = (k & 2) ? w.nx - 1 : 0, y = (k & 1) ? w.ny - 1 : 0;
-      const long long c = (long long)x * w.ny + y;
-      Mom2<R> t = load2<S>(w, N, c, post);
-      auto from_snap = [&](int s) {
-        Mom2<R> m;
-        m.rho = snap[s][0]; m.ux = snap[s][1]; m.uy = snap[s][2];
-        m.sxx = snap[s][3]; m.syy = snap[s][4]; m.sxy = snap[s][5]; m.drho = snap[s][6];
-        return m;
-      };
-      // x face first (left dr 0 / right dr 2), then y face (top dr 1 / bottom dr 3)
-      if (x == 0) t = bc_core<R>(w, 0, t, from_snap(y == 0 ? 0 : 2));
-      else t = bc_core<R>(w, 2, t, load2<S>(w, N, (long long)(w.nx - 2) * w.ny + y, post));
-      if (y == w.ny - 1) t = bc_core<R>(w, 1, t, load2<S>(w, N, (long long)x * w.ny + w.ny - 2, post));
-      else t = bc_core<R>(w, 3, t, x == 0 ? from_snap(1) : from_snap(3));
-      store2<S>(w, N, c, post, t);
+    };
+    if (part == 0 && tid < 32) {
+      __shared__ Mom2<R> old[8];  // ends of the sides x = 0, x = nx - 1, y = ny - 1, y = 0
+      if (tid < 8) {
+        const int side = tid >> 1, base = side < 2 ? side * ey : 2 * ey + (side - 2) * ex;
+        const int last = (side < 2 ? ey : ex) - 1;
+        if (!(tid & 1)) update(base, &old[tid]);
+        else if (last > 0) update(base + last, &old[tid]);
+      }
+      __syncwarp();
+      if (tid < 4) {
+        const int x = (tid & 2) ? w.nx - 1 : 0, y = (tid & 1) ? w.ny - 1 : 0;
+        const long long c = (long long)x * w.ny + y;
+        Mom2<R> t = load2<S>(w, N, c, post);
+        // x face first (left dr 0 / right dr 2), then y face (top dr 1 / bottom dr 3)
+        if (x == 0) t = bc_core<R>(w, 0, t, old[y == 0 ? 6 : 4]);
+        else t = bc_core<R>(w, 2, t, load2<S>(w, N, (long long)(w.nx - 2) * w.ny + y, post));
+        if (y == w.ny - 1) t = bc_core<R>(w, 1, t, load2<S>(w, N, (long long)x * w.ny + w.ny - 2, post));
+        else t = bc_core<R>(w, 3, t, old[x == 0 ? 0 : 2]);
+        store2<S>(w, N, c, post, t);
+      }
+    } else {
+      // the first warp of the first block is not among these
+      const int total = 2 * ey + 2 * ex;
+      for (int k = part * BC_THREADS + tid - 32; k < total; k += BC_BLOCKS * BC_THREADS - 32) {
+        const bool x_side = k < 2 * ey;
+        const int i = x_side ? k % ey : (k - 2 * ey) % ex;
+        if (i > 0 && i < (x_side ? ey : ex) - 1) update(k, nullptr);
+      }
     }
   }
-  for (int s = threadIdx.x; s < w.n_objects; s += blockDim.x) {
-    if (w.force_x) w.force_x[s] = float(w.loads64[3 * s]);
-    if (w.force_y) w.force_y[s] = float(w.loads64[3 * s + 1]);
-    if (w.torque) w.torque[s] = float(w.loads64[3 * s + 2]);
-  }
+  if (part == BC_BLOCKS - 1)
+    for (int s = tid; s < w.n_objects; s += BC_THREADS) {
+      if (w.force_x) w.force_x[s] = float(w.loads64[3 * s]);
+      if (w.force_y) w.force_y[s] = float(w.loads64[3 * s + 1]);
+      if (w.torque) w.torque[s] = float(w.loads64[3 * s + 2]);
+    }
 }
 
 // -------------------------------------------------------------------------- init
@@ -998,7 +1006,7 @@ template <class S> int run_phases(const d2::Launch& L, int n, int maxx, int maxy
     }
   }
   if (phases & HL_PHASE_BC) {
-    d2::boundary_kernel<S><<<n, 512, 0, st>>>(L);
+    d2::boundary_kernel<S><<<dim3(n, d2::BC_BLOCKS), d2::BC_THREADS, 0, st>>>(L);
     HL_LAUNCH_CHECK("d2q9 apply_bc");
   }
   return HL_OK;

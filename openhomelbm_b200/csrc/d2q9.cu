@@ -558,22 +558,27 @@ __device__ Cut get_cutcell(const World& w, float x, float y, float dx, float dy)
   return r;
 }
 
-// get_cutcell over a candidate list: cand[k] = (solid << 16) | segment, in ascending
-// (solid, segment) order, holding every segment of a near solid that can cross a link of the
-// cell. The per-segment arithmetic and the tie rule (first nearest wins) are get_cutcell's, so
-// the result is the same.
-// tf_all / nseg_all: the world's transformed segments [n][max_segments][2] and segment counts
-// (shared-memory copies or the world's own arrays).
-__device__ Cut get_cutcell_list(const float* tf_all, const int* nseg_all, int max_segments, const int* cand, int nc,
-                                float x, float y, float dx, float dy) {
+// Segment j = solid * max_segments + n of a world: its end points (x, y) and (z, w).
+__device__ __forceinline__ float4 segment_of(const World& w, int j) {
+  const int s = j / w.max_segments, n = j - s * w.max_segments;
+  const float* tf = w.tf + size_t(s) * w.max_segments * 2;
+  const int n1 = n + 1 == w.line_num[s] ? 0 : n + 1;
+  return make_float4(tf[2 * n], tf[2 * n + 1], tf[2 * n1], tf[2 * n1 + 1]);
+}
+
+// get_cutcell over a candidate list, segments cand[k] in any order, holding every segment of a near
+// solid that can cross a link of the cell. The per-segment arithmetic is get_cutcell's, and of
+// equally near crossings the lowest segment wins as in its ascending loop, so the result is the same.
+// segs: the world's segments in shared memory, or NULL.
+__device__ __forceinline__ Cut get_cutcell_list(const World& w, const float4* segs, const int* cand, int nc, float x,
+                                                float y, float dx, float dy) {
   Cut r{-1.f, -1.f, -1, -1};
+  int best = 0x7fffffff;
   const float ax = x - dx, ay = y - dy, bx = x, by = y;
   for (int k = 0; k < nc; ++k) {
-    const int s = cand[k] >> 16, n = cand[k] & 0xffff;
-    const int nseg = nseg_all[s];
-    const float* tf = tf_all + size_t(s) * max_segments * 2;
-    const int n1 = n + 1 == nseg ? 0 : n + 1;
-    const float cx = tf[2 * n], cy = tf[2 * n + 1], ex = tf[2 * n1], ey = tf[2 * n1 + 1];
+    const int j = cand[k];
+    const float4 g = segs ? segs[j] : segment_of(w, j);
+    const float cx = g.x, cy = g.y, ex = g.z, ey = g.w;
     const float abc = (ax - cx) * (by - cy) - (ay - cy) * (bx - cx);
     const float abd = (ax - ex) * (by - ey) - (ay - ey) * (bx - ex);
     if (abc * abd >= 0.f) continue;
@@ -581,26 +586,31 @@ __device__ Cut get_cutcell_list(const float* tf_all, const int* nseg_all, int ma
     const float cdb = cda + abc - abd;
     if (cda * cdb > 0.f) continue;
     const float t = 1.f - cda / (abd - abc);
-    if (r.t < 0.f || t < r.t) {
+    if (r.t < 0.f || t < r.t || (t == r.t && j < best)) {
+      best = j;
       r.t = t;
-      r.solid = s;
       r.ratio = abc / (abc - abd);
-      r.seg = n;
     }
+  }
+  if (r.t >= 0.f) {
+    r.solid = best / w.max_segments;
+    r.seg = best - r.solid * w.max_segments;
   }
   return r;
 }
 
-constexpr int MAX_CAND = 24;  // candidate segments kept per cell; more: the full scan
-constexpr int BAND_TF_FLOATS = 4096;  // transformed segment coordinates staged per block
-constexpr int BAND_THREADS = 256, BAND_POOL = 1024;  // candidate segments kept per block and pass
+constexpr int BAND_SEGS = 1024;       // segments staged per block
+constexpr int BAND_THREADS = 128;     // cells of a block's pass
+constexpr int BAND_CAND = 16;         // candidate segments kept per cell; more: the full scan
+constexpr int BAND_BLOCKS = 96;       // blocks per world
 
-// The cells near a solid. Only a few cells of a block lie next to an outline, and a cut cell is a
-// chain of nine links, each a search and a load, so a block works in three passes over its cells:
-// every thread screens one cell and lists it with its candidate segments in shared memory; the
-// threads then take the listed cells' links, one (cell, link) each; and a thread per cut cell
-// collides its nine populations. (A thread per cell through all nine links left 9 threads of a warp
-// active: 37 us for one 96-sided outline, 94 us for 60 worlds of eight; this form 9 and 49.)
+// The cells near a solid. Only a few cells of a block lie next to an outline, and a cut cell is nine
+// links, each a search and a load, so a block takes its cells in three passes: a thread per outline
+// segment notes it with the cells that it passes (a thread per cell looking through all segments
+// was most of the time); the threads then take the noted cells' links, one (cell, link) each; and a
+// thread per cut cell collides its nine populations. A thread per cell through all of it had 9
+// threads of a warp active: 35 us for one 96-sided outline at 512 x 128 and 98 us for 60 worlds of
+// eight 26-sided ones; this form takes 13.6 and 64.
 template <class S> __global__ void __launch_bounds__(BAND_THREADS) band_kernel(const __grid_constant__ Launch L) {
   using R = typename S::R;
   using T = typename S::T;
@@ -616,16 +626,16 @@ template <class S> __global__ void __launch_bounds__(BAND_THREADS) band_kernel(c
   __shared__ double acc[MAX_SOLIDS * 3];
   // the world's per-solid band radii and segments, read by every cell's screening and ray
   // tests: staged in shared memory (the segments when they fit)
-  __shared__ float s_tf[BAND_TF_FLOATS];
+  __shared__ float4 s_seg[BAND_SEGS];
   __shared__ float s_px[MAX_SOLIDS], s_py[MAX_SOLIDS], s_r2[MAX_SOLIDS];
   __shared__ int s_nseg[MAX_SOLIDS];
   __shared__ R s_pop[BAND_THREADS * 9];
-  __shared__ int s_cell[BAND_THREADS], s_first[BAND_THREADS], s_count[BAND_THREADS], s_cut[BAND_THREADS];
-  __shared__ int s_cand[BAND_POOL];
-  __shared__ int n_listed, n_pool, touched;
+  __shared__ int s_cell[BAND_THREADS], s_count[BAND_THREADS], s_cut[BAND_THREADS];
+  __shared__ int s_cand[BAND_THREADS * BAND_CAND];
+  __shared__ int n_listed, touched;
   const int nsol = min(w.n_objects, MAX_SOLIDS);
-  const int n_tf = w.n_objects * w.max_segments * 2;
-  const bool staged = w.n_objects <= MAX_SOLIDS && n_tf <= BAND_TF_FLOATS;
+  const int max_seg = w.max_segments, n_seg = w.n_objects * max_seg;
+  const float4* segs = n_seg <= BAND_SEGS ? s_seg : nullptr;
   for (int k = tid; k < nsol * 3; k += BAND_THREADS) acc[k] = 0.0;
   for (int s = tid; s < nsol; s += BAND_THREADS) {
     const float scale = w.scale[s] * float(w.nx);
@@ -634,56 +644,53 @@ template <class S> __global__ void __launch_bounds__(BAND_THREADS) band_kernel(c
     s_r2[s] = w.max_radius[s] * scale * scale;
     s_nseg[s] = w.line_num[s];
   }
-  if (staged)
-    for (int k = tid; k < n_tf; k += BAND_THREADS) s_tf[k] = w.tf[k];
-  if (tid == 0) n_listed = n_pool = touched = 0;
+  if (segs)
+    for (int j = tid; j < n_seg; j += BAND_THREADS) s_seg[j] = segment_of(w, j);
+  if (tid == 0) n_listed = touched = 0;
+  s_count[tid] = 0;
   __syncthreads();
-  const float* tfb = staged ? s_tf : w.tf;
   const long long N = (long long)w.nx * w.ny;
   const T* cur = static_cast<const T*>(cur_of(L, w));
   for (long long k0 = (long long)blockIdx.x * BAND_THREADS; k0 < area; k0 += (long long)gridDim.x * BAND_THREADS) {
-    // 1. screen. The segments of the near solids (get_cutcell's radius test) that can cross a link
-    // of the cell: every link lies in the square [x-1, x+1] x [y-1, y+1], so a segment whose box
-    // misses that square widened by 1e-3 crosses none. No candidate: no cut link, and the stream
-    // kernel's value is already the cell's update.
-    const long long k = k0 + tid;
-    const int x = x0 + int(k / bw), y = y0 + int(k % bw);
-    if (k < area && is_fluid(w, x, y, (long long)x * w.ny + y)) {
-      int cand[MAX_CAND];
-      int nc = 0;
-      bool overflow = false;
-      const float fxc = float(x), fyc = float(y);
-      for (int s = 0; s < nsol; ++s) {
-        const int nseg = s_nseg[s];
-        if (nseg <= 0) continue;
-        const float px = fxc - s_px[s], py = fyc - s_py[s];
-        if (px * px + py * py > s_r2[s]) continue;
-        const float* tf = tfb + size_t(s) * w.max_segments * 2;
-        float cx = tf[0], cy = tf[1];
-        for (int n = 0; n < nseg; ++n) {  // segment n: point n to point n + 1
-          const int n1 = n + 1 == nseg ? 0 : n + 1;
-          const float ex = tf[2 * n1], ey = tf[2 * n1 + 1];
-          const bool hit = !(fmaxf(cx, ex) < fxc - 1.001f || fminf(cx, ex) > fxc + 1.001f ||
-                             fmaxf(cy, ey) < fyc - 1.001f || fminf(cy, ey) > fyc + 1.001f);
-          cx = ex;
-          cy = ey;
-          if (!hit) continue;
-          if (nc < MAX_CAND) cand[nc++] = (s << 16) | n;
-          else overflow = true;
+    // 1. The segments of the near solids (get_cutcell's radius test) that can cross a link of a
+    // cell: every link lies in the square [x-1, x+1] x [y-1, y+1], so a segment whose box misses that
+    // square widened by 1e-3 crosses none. No candidate: no cut link, and the stream kernel's value
+    // is already the cell's update. The pass's cells are rows xa .. xb of the box, clipped.
+    const int k_end = int(area - k0 < BAND_THREADS ? area - k0 : BAND_THREADS);
+    const int xa = x0 + int(k0 / bw), ya = y0 + int(k0 % bw);  // the pass's first and last cell
+    const int xb = x0 + int((k0 + k_end - 1) / bw), yb = y0 + int((k0 + k_end - 1) % bw);
+    for (int j = tid; j < 4 * n_seg; j += BAND_THREADS) {  // four threads a segment, every fourth row each
+      const int id = j >> 2, s = id / max_seg;
+      if (id - s * max_seg >= s_nseg[s]) continue;
+      const float4 g = segs ? segs[id] : segment_of(w, id);
+      const float cx = g.x, cy = g.y, ex = g.z, ey = g.w;
+      const float hx = fmaxf(cx, ex), lx = fminf(cx, ex), hy = fmaxf(cy, ey), ly = fminf(cy, ey);
+      // cells outside this range fail the exact test below (it is wider by up to one; fmaxf / fminf
+      // drop a NaN, and the clips bound the rest)
+      const int i0 = int(fminf(fmaxf(floorf(lx - 1.01f), float(xa)), float(xb + 1)));
+      const int i1 = int(fmaxf(fminf(ceilf(hx + 1.01f), float(xb)), float(xa - 1)));
+      const int j0 = int(fminf(fmaxf(floorf(ly - 1.01f), float(y0)), float(y1 + 1)));
+      const int j1 = int(fmaxf(fminf(ceilf(hy + 1.01f), float(y1)), float(y0 - 1)));
+      for (int x = i0 + (j & 3); x <= i1; x += 4) {
+        const int ye = x == xb ? min(j1, yb) : j1;
+        for (int y = x == xa ? max(j0, ya) : j0; y <= ye; ++y) {
+          const int at = (x - xa) * bw + y - ya;
+          const float fxc = float(x), fyc = float(y);
+          if (hx < fxc - 1.001f || lx > fxc + 1.001f || hy < fyc - 1.001f || ly > fyc + 1.001f) continue;
+          const float px = fxc - s_px[s], py = fyc - s_py[s];
+          if (px * px + py * py > s_r2[s]) continue;
+          const int c = atomicAdd(&s_count[at], 1);
+          if (c < BAND_CAND) s_cand[at * BAND_CAND + c] = id;
         }
       }
-      if (nc > 0) {
-        const int slot = atomicAdd(&n_listed, 1);
-        const int first = overflow ? 0 : atomicAdd(&n_pool, nc);
-        if (!overflow && first + nc <= BAND_POOL) {
-          for (int j = 0; j < nc; ++j) s_cand[first + j] = cand[j];
-        } else {
-          overflow = true;
-        }
-        s_cell[slot] = tid;
-        s_first[slot] = first;
-        s_count[slot] = overflow ? -1 : nc;
-        s_cut[slot] = 0;
+    }
+    __syncthreads();
+    {
+      const long long k = k0 + tid;
+      const int x = x0 + int(k / bw), y = y0 + int(k % bw);
+      if (tid < k_end && s_count[tid] > 0 && is_fluid(w, x, y, (long long)x * w.ny + y)) {
+        s_cell[atomicAdd(&n_listed, 1)] = tid;
+        s_cut[tid] = 0;
       }
     }
     __syncthreads();
@@ -694,8 +701,8 @@ template <class S> __global__ void __launch_bounds__(BAND_THREADS) band_kernel(c
       int hit_solid = -1;
       double lf[3] = {0.0, 0.0, 0.0};
       if (it < listed * 9) {
-        const int slot = it / 9, i = it % 9;
-        const long long kc = k0 + s_cell[slot];
+        const int i = it / listed, at = s_cell[it - i * listed];  // a warp's lanes share directions
+        const long long kc = k0 + at;
         const int cx = x0 + int(kc / bw), cy = y0 + int(kc % bw);
         const int dx = cx_of(i), dy = cy_of(i);
         int xn = cx - dx, yn = cy - dy;
@@ -706,19 +713,19 @@ template <class S> __global__ void __launch_bounds__(BAND_THREADS) band_kernel(c
         R pop = -w2<R>(i);
         if (xn >= 0 && xn < w.nx && yn >= 0 && yn < w.ny) {
           const Mom2<R> mn = load2<S>(w, N, (long long)xn * w.ny + yn, cur);  // the upwind neighbour
-          const int nc = s_count[slot];
-          const Cut cc = nc < 0 ? get_cutcell(w, float(cx), float(cy), float(dx), float(dy))
-                                : get_cutcell_list(tfb, s_nseg, w.max_segments, s_cand + s_first[slot], nc, float(cx),
-                                                   float(cy), float(dx), float(dy));
+          const int nc = s_count[at];
+          const Cut cc = nc > BAND_CAND ? get_cutcell(w, float(cx), float(cy), float(dx), float(dy))
+                                        : get_cutcell_list(w, segs, s_cand + at * BAND_CAND, nc, float(cx), float(cy),
+                                                           float(dx), float(dy));
           if (cc.t >= 0.f && cc.solid >= 0) {
             const Mom2<R> me = load2<S>(w, N, (long long)cx * w.ny + cy, cur);
-            s_cut[slot] = 1;
+            s_cut[at] = 1;
             const int s = cc.solid, nseg = s_nseg[s];
             const int n1 = cc.seg + 1 == nseg ? 0 : cc.seg + 1;
-            const float* tf = tfb + size_t(s) * w.max_segments * 2;
-            const float* tl = w.tf_last + size_t(s) * w.max_segments * 2;
-            const float pcx = tf[2 * cc.seg] + (tf[2 * n1] - tf[2 * cc.seg]) * cc.ratio;
-            const float pcy = tf[2 * cc.seg + 1] + (tf[2 * n1 + 1] - tf[2 * cc.seg + 1]) * cc.ratio;
+            const float4 g = segs ? segs[s * max_seg + cc.seg] : segment_of(w, s * max_seg + cc.seg);
+            const float* tl = w.tf_last + size_t(s) * max_seg * 2;
+            const float pcx = g.x + (g.z - g.x) * cc.ratio;
+            const float pcy = g.y + (g.w - g.y) * cc.ratio;
             const float plx = tl[2 * cc.seg] + (tl[2 * n1] - tl[2 * cc.seg]) * cc.ratio;
             const float ply = tl[2 * cc.seg + 1] + (tl[2 * n1 + 1] - tl[2 * cc.seg + 1]) * cc.ratio;
             const R upx = R((pcx - plx) / w.time_step), upy = R((pcy - ply) / w.time_step);
@@ -744,7 +751,7 @@ template <class S> __global__ void __launch_bounds__(BAND_THREADS) band_kernel(c
             pop = feq_dev_clamped<R>(mn, i);
           }
         }
-        s_pop[slot * 9 + i] = pop;
+        s_pop[at * 9 + i] = pop;
       }
       // the loads of the warp's cut links, summed per solid
       for (unsigned left = __ballot_sync(FULL, hit_solid >= 0); left; left = __ballot_sync(FULL, hit_solid >= 0)) {
@@ -763,17 +770,18 @@ template <class S> __global__ void __launch_bounds__(BAND_THREADS) band_kernel(c
     }
     __syncthreads();
     // 3. the cut cells (the others keep the stream kernel's value: it is already their update)
-    if (tid < listed && s_cut[tid]) {
-      const long long kc = k0 + s_cell[tid];
-      const long long c = (long long)(x0 + int(kc / bw)) * w.ny + y0 + int(kc % bw);
+    if (tid < listed && s_cut[s_cell[tid]]) {
+      const int at = s_cell[tid];
+      const long long c = (long long)(x0 + int((k0 + at) / bw)) * w.ny + y0 + int((k0 + at) % bw);
       R pop[9];
 #pragma unroll
-      for (int i = 0; i < 9; ++i) pop[i] = s_pop[tid * 9 + i];
+      for (int i = 0; i < 9; ++i) pop[i] = s_pop[at * 9 + i];
       const R Fx = w.fx ? R(w.fx[c]) : R(0), Fy = w.fy ? R(w.fy[c]) : R(0);
       store2<S>(w, N, c, static_cast<T*>(post_of(L, w)), collide<R>(pop, Fx, Fy, omega_of<R>(w.vis_shear)));
     }
     __syncthreads();
-    if (tid == 0) n_listed = n_pool = 0;
+    if (tid == 0) n_listed = 0;
+    s_count[tid] = 0;
     __syncthreads();
   }
   if (touched)
@@ -1058,7 +1066,7 @@ template <class S> int run_phases(const d2::Launch& L, int n, int maxx, int maxy
       HL_LAUNCH_CHECK("d2q9 stream_and_collide");
     }
     if (any_solid) {
-      d2::band_kernel<S><<<dim3(64, n), d2::BAND_THREADS, 0, st>>>(L);
+      d2::band_kernel<S><<<dim3(d2::BAND_BLOCKS, n), d2::BAND_THREADS, 0, st>>>(L);
       HL_LAUNCH_CHECK("d2q9 cut-cell band");
     }
   }

@@ -46,3 +46,44 @@ def test_two_steps_match_the_binary64_oracle(nx, ny, bc):
                              dtype=np.float64)
         m, p = new, m
     assert np.abs(f.cur.double().cpu().numpy() - m).max() <= 200 * 2.0 ** -24
+
+
+@pytest.mark.parametrize("n_solids,n_seg,radius", [(1, 3, 5.0), (2, 40, 6.0), (1, 400, 4.0), (5, 230, 6.0)])
+def test_cut_links_of_few_and_many_segments(n_solids, n_seg, radius):
+    """Outlines with few, many (more candidate segments per cell than a block keeps) and very many
+    segments (more than a block stages), moving, two steps against the binary32 oracle, which takes
+    the same cut-link decisions. Tolerance: both sides round, 2 x 200 eps a step, and the loads are
+    sums of at most 600 links of magnitude below 1: 600 x 200 eps."""
+    from openhomelbm_b200.lbm import LBM_Solver
+
+    nx, ny = 90, 64
+    s = LBM_Solver(nx, ny, solid_num=n_solids, use_graph=False)
+    f = s.flows[0]
+    f.vis_shear = 0.05
+    f.bc_type = [0, 1, 1, 1]
+    f.bc_value = np.array([[0.03, 0.0], [0, 0], [0, 0], [0, 0]], np.float32)
+    m, p = _state(nx, ny, 3), _state(nx, ny, 4)
+    f.moments[0].copy_(torch.tensor(m))
+    f.moments[1].copy_(torch.tensor(p))
+    th = np.linspace(0, 2 * np.pi, n_seg, endpoint=False) + 0.1
+    poly = np.stack([np.cos(th), 0.8 * np.sin(th)], 1).astype(np.float32)
+    pos = np.array([[14.3 + 15.1 * k, 30.7 + 1.3 * k] for k in range(n_solids)], np.float32)
+    for k in range(n_solids):
+        f.configure_solid(k, poly, tuple(pos[k]), scale=radius / nx)
+    sol = orc.Solids2D(line=np.stack([poly] * n_solids), line_num=np.full(n_solids, n_seg), position=pos.copy(),
+                       angle=np.zeros(n_solids), scale=np.full(n_solids, np.float32(radius / nx)),
+                       mass_center=np.zeros((n_solids, 2)),
+                       max_radius=f.solid_max_radius.cpu().numpy()).cast(np.float32)
+    eps = 2.0 ** -24
+    for step in range(2):
+        for k in range(n_solids):
+            f.solid_position[k] += torch.tensor([0.02, -0.01], device=f.device)
+            sol.position[k] += np.array([0.02, -0.01], np.float32)
+        s.step()
+        new, loads = orc.step_2d(m, p, vis_shear=np.float32(0.05), bc_type=f.bc_type, bc_value=f.bc_value,
+                                 flag=orc.border_flags_2d(nx, ny), solids=sol)
+        m, p = new, m
+        assert np.abs(f.cur.cpu().numpy() - m).max() <= (step + 1) * 400 * eps
+        got = np.stack([f.solid_forcex.cpu().numpy(), f.solid_forcey.cpu().numpy()], 1)
+        assert np.abs(got).max() > 0
+        assert np.abs(got - loads[:, :2]).max() <= 600 * 200 * eps

@@ -12,6 +12,15 @@
 //   wave 2: cells on two faces (edges), reading snapshots for low faces and wave-1 results
 //           for high faces; the cell next to each low-end corner saves its old value;
 //   wave 3: the 8 corners, likewise.
+// Where every side has at least four cells one launch does all of it (pass_* below): every border
+// cell has one owner. A face cell reads only the cell inside it, so a face's inner cells are
+// independent; an edge's thread also owns the two face cells beside it, whose old and new values the
+// edge reads, and a warp per corner owns the corner, the three edge ends next to it and the three face
+// cells next to those. Old values are read by their owner before it writes. Small worlds are bound by
+// the launches and the chain of loads behind each, large ones by the partial sectors of the z faces.
+// Waves / one pass, us: 64^3 binary32 17.8 / 6.7, 128^3 23.0 / 12.1, 192^3 binary16 37.4 / 25.2, 256^3
+// binary32 85.3 / 78.4, 512^3 bfloat16 363 / 332. The waves remain for sides of three cells, where a
+// face cell lies next to two edges.
 // Face numbering is the reference's: 0 x=0, 1 x=nx-1, 2 y=ny-1, 3 y=0, 4 z=nz-1, 5 z=0.
 
 #include <algorithm>
@@ -70,10 +79,26 @@ template <class S> __device__ __forceinline__ void copy_raw(const BcArgs& a, lon
 #pragma unroll
   for (int k = 0; k < 10; ++k) dst[k] = p[k * a.N + i];
 }
+template <class S> __device__ __forceinline__ void encode_cell(const Mom3<typename S::R>& m, const Scale& sc, typename S::R raw[10]) {
+  if constexpr (S::kEncoded) {
+    raw[0] = m.drho;
+    raw[1] = m.ux * sc.inv_u;
+    raw[2] = m.uy * sc.inv_u;
+    raw[3] = m.uz * sc.inv_u;
+    raw[4] = fmaf(-m.ux, m.ux, m.sxx) * sc.inv_s;
+    raw[5] = fmaf(-m.uy, m.uy, m.syy) * sc.inv_s;
+    raw[6] = fmaf(-m.uz, m.uz, m.szz) * sc.inv_s;
+    raw[7] = fmaf(-m.ux, m.uy, m.sxy) * sc.inv_s;
+    raw[8] = fmaf(-m.ux, m.uz, m.sxz) * sc.inv_s;
+    raw[9] = fmaf(-m.uy, m.uz, m.syz) * sc.inv_s;
+  } else {
+    encode3<S>(m, sc, raw);
+  }
+}
 template <class S> __device__ __forceinline__ void store_cell(const BcArgs& a, long long i, const Mom3<typename S::R>& m) {
   typename S::T* p = static_cast<typename S::T*>(a.post);
   typename S::R raw[10];
-  encode3<S>(m, a.sc, raw);
+  encode_cell<S>(m, a.sc, raw);
 #pragma unroll
   for (int k = 0; k < 10; ++k) p[k * a.N + i] = S::from_r(raw[k], unsigned(k * a.N + i));
 }
@@ -84,15 +109,15 @@ template <class S> __device__ __forceinline__ void store_cell(const BcArgs& a, l
 // sum w c_a c_b = delta_ab / 3, odd moments 0 and sum w c_a c_b c_c c_d = (delta_ab delta_cd +
 // delta_ac delta_bd + delta_ad delta_bc) / 9, so P_ab = (rho - 1) delta_ab / 3 + rho u_a u_b
 // and S_ab = u_a u_b exactly: computed in that closed form, not as the reference's 27-term
-// binary32 sums (which agree with it to their rounding). out = xx, yy, zz, xy, xz, yz.
-template <class R> __device__ __forceinline__ void feq_s(R ux, R uy, R uz, R out[6]) {
-  out[0] = ux * ux;
-  out[1] = uy * uy;
-  out[2] = uz * uz;
-  out[3] = ux * uy;
-  out[4] = ux * uz;
-  out[5] = uy * uz;
-}
+// binary32 sums (which agree with it to their rounding).
+// The products are fused explicitly, here and in encode_cell, so that every kernel that computes a
+// cell gets the same bits (16-bit storages draw their rounding noise from them).
+__device__ __forceinline__ float fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+// the equilibrium's stress difference between velocities a and b, one component
+template <class R> __device__ __forceinline__ R feq_gap(R a1, R a2, R b1, R b2) { return fma_rn(a1, a2, -mul_rn(b1, b2)); }
 
 // apply_bc_core_3d (envs/lbm3d/lbm_func_3d.py:627-648): new state of boundary cell t from
 // its own old state and its inward neighbour nb.
@@ -109,15 +134,12 @@ template <class R> __device__ Mom3<R> bc_core(const BcArgs& a, int dr, const Mom
   }
   r.rho = nb.rho;
   r.drho = nb.drho;
-  R sc[6], sb[6];
-  feq_s<R>(r.ux, r.uy, r.uz, sc);
-  feq_s<R>(nb.ux, nb.uy, nb.uz, sb);
-  r.sxx = sc[0] - sb[0] + nb.sxx;
-  r.syy = sc[1] - sb[1] + nb.syy;
-  r.szz = sc[2] - sb[2] + nb.szz;
-  r.sxy = sc[3] - sb[3] + nb.sxy;
-  r.sxz = sc[4] - sb[4] + nb.sxz;
-  r.syz = sc[5] - sb[5] + nb.syz;
+  r.sxx = feq_gap(r.ux, r.ux, nb.ux, nb.ux) + nb.sxx;
+  r.syy = feq_gap(r.uy, r.uy, nb.uy, nb.uy) + nb.syy;
+  r.szz = feq_gap(r.uz, r.uz, nb.uz, nb.uz) + nb.szz;
+  r.sxy = feq_gap(r.ux, r.uy, nb.ux, nb.uy) + nb.sxy;
+  r.sxz = feq_gap(r.ux, r.uz, nb.ux, nb.uz) + nb.sxz;
+  r.syz = feq_gap(r.uy, r.uz, nb.uy, nb.uz) + nb.syz;
   return r;
 }
 
@@ -210,6 +232,151 @@ template <class S> __device__ __forceinline__ void wave3_corner(const BcArgs& a,
   store_cell<S>(a, i, t);
 }
 
+// ---------------------------------------------------------------- one pass
+// A cell's stored planes, as they are and decoded.
+template <class S> struct Cell {
+  typename S::T v[10];
+  __device__ __forceinline__ void load(const BcArgs& a, long long i) { copy_raw<S>(a, i, v); }
+  __device__ __forceinline__ void store(const BcArgs& a, long long i) const {
+    typename S::T* p = static_cast<typename S::T*>(a.post);
+#pragma unroll
+    for (int k = 0; k < 10; ++k) p[k * a.N + i] = v[k];
+  }
+  __device__ __forceinline__ Mom3<typename S::R> moments(const BcArgs& a) const { return load_slot<S>(a, v); }
+  __device__ __forceinline__ void set(const BcArgs& a, long long i, const Mom3<typename S::R>& m) {  // as store_cell
+    typename S::R raw[10];
+    encode_cell<S>(m, a.sc, raw);
+#pragma unroll
+    for (int k = 0; k < 10; ++k) v[k] = S::from_r(raw[k], unsigned(k * a.N + i));
+  }
+};
+
+// The new value of a cell on face (ax, side) alone. Its own old value matters only to conditions
+// that neither set nor copy the velocity.
+template <class S> __device__ __forceinline__ Mom3<typename S::R> face_value(const BcArgs& a, int ax, int side, const int cell[3]) {
+  int nbr[3] = {cell[0], cell[1], cell[2]};
+  nbr[ax] = side ? a.n[ax] - 2 : 1;
+  const int dr = face_dr(ax, side);
+  const auto n = load_cell<S>(a, lin(a, nbr));
+  const auto t = a.bc_type[dr] == 0 || a.bc_type[dr] == 1 ? n : load_cell<S>(a, lin(a, cell));
+  return bc_core(a, dr, t, n);
+}
+
+template <class S> __device__ __forceinline__ void pass_face(const BcArgs& a, int fid, long long first, long long stride) {
+  const int ax = fid >> 1, side = fid & 1;
+  const int b = ax == 0 ? 1 : 0, c = ax == 2 ? 1 : 2;
+  const int nb = a.n[b] - 4, nc = a.n[c] - 4;  // without the cells beside the edges
+  if (nb <= 0 || nc <= 0) return;
+  const long long total = (long long)nb * nc;
+  for (long long k = first; k < total; k += stride) {
+    int cell[3];
+    cell[ax] = side ? a.n[ax] - 1 : 0;
+    cell[b] = 2 + int(k / nc);
+    cell[c] = 2 + int(k % nc);
+    store_cell<S>(a, lin(a, cell), face_value<S>(a, ax, side, cell));
+  }
+}
+
+// Edge cell `pos` (2 .. n - 3) of edge eid and the two face cells beside it.
+template <class S> __device__ __forceinline__ void pass_edge(const BcArgs& a, int eid, int pos) {
+  const int a3 = eid >> 2, sd[2] = {(eid >> 1) & 1, eid & 1};
+  const int af[2] = {a3 == 0 ? 1 : 0, a3 == 2 ? 1 : 2};
+  int cell[3];
+  cell[a3] = pos;
+  for (int f = 0; f < 2; ++f) cell[af[f]] = sd[f] ? a.n[af[f]] - 1 : 0;
+  auto t = load_cell<S>(a, lin(a, cell));
+  Cell<S> fresh[2];
+  long long at[2];
+#pragma unroll
+  for (int f = 0; f < 2; ++f) {
+    // the neighbour through face f lies on the other face
+    int rim[3] = {cell[0], cell[1], cell[2]};
+    rim[af[f]] = sd[f] ? a.n[af[f]] - 2 : 1;
+    at[f] = lin(a, rim);
+    Cell<S> old;
+    old.load(a, at[f]);
+    fresh[f].set(a, at[f], face_value<S>(a, af[1 - f], sd[1 - f], rim));
+    t = bc_core(a, face_dr(af[f], sd[f]), t, (sd[f] == 0 ? old : fresh[f]).moments(a));
+  }
+  fresh[0].store(a, at[0]);
+  fresh[1].store(a, at[1]);
+  store_cell<S>(a, lin(a, cell), t);
+}
+
+// Corner `corner` (bits x, y, z sides) by one warp: lane q < 3 the face cell next to it on face q and
+// the edge end along axis q; buf: this warp's old and new values of those.
+template <class S> struct CornerBuf {
+  Cell<S> face_old[3], face_new[3], edge_old[3], edge_new[3];
+};
+template <class S> __device__ __forceinline__ void pass_corner(const BcArgs& a, int corner, int lane, CornerBuf<S>& buf) {
+  const int sd[3] = {(corner >> 2) & 1, (corner >> 1) & 1, corner & 1};
+  int border[3], inner[3];
+#pragma unroll
+  for (int q = 0; q < 3; ++q) {
+    border[q] = sd[q] ? a.n[q] - 1 : 0;
+    inner[q] = sd[q] ? a.n[q] - 2 : 1;
+  }
+  long long face_at = 0, edge_at = 0;
+  if (lane < 3) {
+    int fc[3] = {inner[0], inner[1], inner[2]}, ec[3] = {border[0], border[1], border[2]};
+    fc[lane] = border[lane];
+    ec[lane] = inner[lane];
+    face_at = lin(a, fc);
+    edge_at = lin(a, ec);
+    buf.face_old[lane].load(a, face_at);
+    buf.edge_old[lane].load(a, edge_at);
+    buf.face_new[lane].set(a, face_at, face_value<S>(a, lane, sd[lane], fc));
+  }
+  __syncwarp();
+  if (lane < 3) {
+    const int o1 = lane == 0 ? 1 : 0, o2 = lane == 2 ? 1 : 2;
+    // the neighbour through face o1 lies on face o2 and the other way round
+    auto t = buf.edge_old[lane].moments(a);
+    t = bc_core(a, face_dr(o1, sd[o1]), t, (sd[o1] == 0 ? buf.face_old[o2] : buf.face_new[o2]).moments(a));
+    t = bc_core(a, face_dr(o2, sd[o2]), t, (sd[o2] == 0 ? buf.face_old[o1] : buf.face_new[o1]).moments(a));
+    buf.edge_new[lane].set(a, edge_at, t);
+  }
+  __syncwarp();
+  if (lane == 0) {
+    const long long i = lin(a, border);
+    auto t = load_cell<S>(a, i);
+#pragma unroll
+    for (int ax = 0; ax < 3; ++ax)
+      t = bc_core(a, face_dr(ax, sd[ax]), t, (sd[ax] == 0 ? buf.edge_old[ax] : buf.edge_new[ax]).moments(a));
+    store_cell<S>(a, i, t);
+  }
+  if (lane < 3) {
+    buf.face_new[lane].store(a, face_at);
+    buf.edge_new[lane].store(a, edge_at);
+  }
+}
+
+// Block row 0: the corners (a warp each, block 0) and the edges; rows 1 .. 6: the faces.
+constexpr int PASS_THREADS = 128;
+template <class S> __device__ __forceinline__ void one_pass(const BcArgs& a) {
+  if (blockIdx.y > 0) {
+    pass_face<S>(a, blockIdx.y - 1, blockIdx.x * (long long)PASS_THREADS + threadIdx.x, (long long)gridDim.x * PASS_THREADS);
+  } else if (blockIdx.x < 2) {
+    __shared__ CornerBuf<S> buf[PASS_THREADS / 32];
+    const int warp = threadIdx.x >> 5;
+    pass_corner<S>(a, int(blockIdx.x) * (PASS_THREADS / 32) + warp, threadIdx.x & 31, buf[warp]);
+  } else {
+    for (int k = (blockIdx.x - 2) * PASS_THREADS + threadIdx.x; k < 12 * a.maxn; k += (gridDim.x - 2) * PASS_THREADS) {
+      const int eid = k / a.maxn, pos = k - eid * a.maxn;
+      if (pos >= 2 && pos < a.n[eid >> 2] - 2) pass_edge<S>(a, eid, pos);
+    }
+  }
+}
+template <class S> __global__ void __launch_bounds__(PASS_THREADS) pass_kernel(const __grid_constant__ BcArgs a) { one_pass<S>(a); }
+template <class S> __global__ void __launch_bounds__(PASS_THREADS) pass_batch_kernel(const BcArgs* __restrict__ args, int parity) {
+  one_pass<S>(args[2 * blockIdx.z + parity]);
+}
+// blocks per row: a thread per face cell (grid-stride beyond 2048 blocks), at least four
+int pass_blocks(int maxn) {
+  const long long g = ((long long)maxn * maxn + PASS_THREADS - 1) / PASS_THREADS;
+  return int(g > 2048 ? 2048 : g < 4 ? 4 : g);
+}
+
 // One world: blockIdx.y = face / edge.
 template <class S> __global__ void wave1_kernel(const BcArgs a) {
   wave1_face<S>(a, blockIdx.y, blockIdx.x * (long long)blockDim.x + threadIdx.x, (long long)gridDim.x * blockDim.x);
@@ -259,6 +426,11 @@ int wave1_blocks(int maxn) {
 
 template <class S> int launch_bc(const hl_world3d* w, const hl_bc3d* bc, void* scratch, cudaStream_t st) {
   const BcArgs a = make_bc_args(w, bc, scratch);
+  if (w->nx >= 4 && w->ny >= 4 && w->nz >= 4) {
+    pass_kernel<S><<<dim3(pass_blocks(a.maxn), 7), PASS_THREADS, 0, st>>>(a);
+    HL_LAUNCH_CHECK("d3q27 apply_bc");
+    return HL_OK;
+  }
   wave1_kernel<S><<<dim3(wave1_blocks(a.maxn), 6), 256, 0, st>>>(a);
   HL_LAUNCH_CHECK("d3q27 apply_bc wave 1");
   wave2_kernel<S><<<dim3((a.maxn + 127) / 128, 12), 128, 0, st>>>(a);
@@ -272,12 +444,17 @@ template <class S> int launch_bc(const hl_world3d* w, const hl_bc3d* bc, void* s
 struct BcBatchInfo {
   int n;
   hl_dtype dtype;
-  int maxn;
+  int maxn, minn;
 };
 std::mutex g_bcb_mu;
 std::map<const void*, BcBatchInfo> g_bcb;
 
 template <class S> int launch_bc_batch(const BcArgs* args, const BcBatchInfo& b, int parity, cudaStream_t st) {
+  if (b.minn >= 4) {
+    pass_batch_kernel<S><<<dim3(pass_blocks(b.maxn), 7, b.n), PASS_THREADS, 0, st>>>(args, parity);
+    HL_LAUNCH_CHECK("d3q27 apply_bc batch");
+    return HL_OK;
+  }
   wave1_batch_kernel<S><<<dim3(wave1_blocks(b.maxn), 6, b.n), 256, 0, st>>>(args, parity);
   HL_LAUNCH_CHECK("d3q27 apply_bc batch wave 1");
   wave2_batch_kernel<S><<<dim3((b.maxn + 127) / 128, 12, b.n), 128, 0, st>>>(args, parity);
@@ -420,7 +597,7 @@ extern "C" int hl_d3q27_bc_batch_prepare(const hl_world3d* worlds, const hl_bc3d
   HL_CHECK_ARG(reinterpret_cast<uintptr_t>(desc) % 16 == 0, "apply_bc_3d batch: desc not 16-byte aligned");
   const hl_dtype dtype = worlds[0].storage.dtype;
   std::vector<d3bc::BcArgs> host(size_t(2) * n_domains);
-  int maxn = 0;
+  int maxn = 0, minn = 1 << 30;
   for (int i = 0; i < n_domains; ++i) {
     const hl_world3d& w = worlds[i];
     HL_CHECK_ARG(!w.periodic, "apply_bc_3d batch: world %d is periodic (no boundary pass)", i);
@@ -434,13 +611,14 @@ extern "C" int hl_d3q27_bc_batch_prepare(const hl_world3d* worlds, const hl_bc3d
     a.post = const_cast<void*>(w.cur);
     host[2 * i + 1] = a;
     maxn = std::max(maxn, a.maxn);
+    minn = std::min(minn, std::min(w.nx, std::min(w.ny, w.nz)));
   }
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   cudaError_t e = cudaMemcpyAsync(desc, host.data(), bytes, cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);  // host staging buffer ends here
   if (e != cudaSuccess) return cuda_status(e, "apply_bc_3d batch: descriptor upload");
   std::lock_guard<std::mutex> lock(d3bc::g_bcb_mu);
-  d3bc::g_bcb[desc] = d3bc::BcBatchInfo{n_domains, dtype, maxn};
+  d3bc::g_bcb[desc] = d3bc::BcBatchInfo{n_domains, dtype, maxn, minn};
   return HL_OK;
 }
 

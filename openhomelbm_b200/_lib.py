@@ -212,8 +212,11 @@ def ptr(t):
 def stream_ptr(stream=None):
     import torch
 
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return c_void_p(s.cuda_stream)
+    if stream is not None:
+        return c_void_p(stream.cuda_stream)
+    if torch.cuda.is_initialized():  # the current stream's handle without building a Stream object
+        return c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
+    return c_void_p(torch.cuda.current_stream().cuda_stream)
 
 
 DTYPES = {"float32": HL_F32, "float16": HL_F16, "bfloat16": HL_BF16, "float64": HL_F64}

@@ -17,14 +17,15 @@ from . import _lib
 
 
 def _dev(t, dtype, shape=None, name="buffer"):
-    t = torch.as_tensor(t)
+    if type(t) is not torch.Tensor:
+        t = torch.as_tensor(t)
     if not t.is_cuda:
         raise ValueError(f"{name} must be a CUDA tensor")
     if t.dtype != dtype:
         raise ValueError(f"{name} must be {dtype}, got {t.dtype}")
     if not t.is_contiguous():
         raise ValueError(f"{name} must be contiguous")
-    if shape is not None and tuple(t.shape) != tuple(shape):
+    if shape is not None and t.shape != shape:
         raise ValueError(f"{name} has shape {tuple(t.shape)}, expected {tuple(shape)}")
     return t
 
@@ -58,17 +59,37 @@ def _solver(x):
     return x.solver if isinstance(x, FlowArray) else x
 
 
+def _on(solver, t):
+    if type(t) is torch.Tensor and t.device == solver.solid_position_all.device:
+        return t
+    return torch.as_tensor(t, device=solver.device)
+
+
+# The arrays of finalize_mappings have the layout the kernels read: those pass without the chain of
+# tensor operations (a few us of host time each) that brings another layout or type into it.
+def _rows(t, nsel, dim, name):
+    if not (type(t) is torch.Tensor and t.dtype == torch.float32 and t.shape == (nsel, dim) and t.is_contiguous()):
+        t = t.to(torch.float32).reshape(nsel, -1)[:, :dim].contiguous()
+    return _dev(t, torch.float32, (nsel, dim), name)
+
+
+def _flat(t, nsel):
+    if not (type(t) is torch.Tensor and t.dtype == torch.float32 and t.shape == (nsel,) and t.is_contiguous()):
+        t = t.to(torch.float32).reshape(nsel).contiguous()
+    return _dev(t, torch.float32, (nsel,), "scales")
+
+
 def _mapping(solver, solid_ids, mujoco_origins, lbm_origins, scales, dim):
     ids = _ids(solid_ids if solid_ids is not None else solver.solid_ids_wp, solver.solid_num, "solid_ids")
     nsel = ids.numel()
-    mo = solver.mujoco_origins_wp if mujoco_origins is None else torch.as_tensor(mujoco_origins, device=solver.device)
-    lo = solver.lbm_origins_wp if lbm_origins is None else torch.as_tensor(lbm_origins, device=solver.device)
-    sc = solver.scales_wp if scales is None else torch.as_tensor(scales, device=solver.device)
+    mo = solver.mujoco_origins_wp if mujoco_origins is None else _on(solver, mujoco_origins)
+    lo = solver.lbm_origins_wp if lbm_origins is None else _on(solver, lbm_origins)
+    sc = solver.scales_wp if scales is None else _on(solver, scales)
     if mo is None or lo is None or sc is None:
         raise ValueError("coordinate mappings are missing: call finalize_mappings or pass them")
-    mo = _dev(mo.to(torch.float32).reshape(nsel, -1)[:, :dim].contiguous(), torch.float32, (nsel, dim), "mujoco_origins")
-    lo = _dev(lo.to(torch.float32).reshape(nsel, -1)[:, :dim].contiguous(), torch.float32, (nsel, dim), "lbm_origins")
-    sc = _dev(sc.to(torch.float32).reshape(nsel).contiguous(), torch.float32, (nsel,), "scales")
+    mo = _rows(mo, nsel, dim, "mujoco_origins")
+    lo = _rows(lo, nsel, dim, "lbm_origins")
+    sc = _flat(sc, nsel)
     return ids, nsel, mo, lo, sc
 
 
@@ -111,8 +132,7 @@ def _loads(mode, solver, solid_ids, scales, fconv, tconv, forces_out, torques_ou
     nsel, W = ids.numel(), solver.nworld
     fo = _dev(forces_out, torch.float32, (W, nsel, 3), "forces_out")
     to = _dev(torques_out, torch.float32, (W, nsel, 3), "torques_out")
-    sc = None if scales is None else _dev(torch.as_tensor(scales, device=solver.device).to(torch.float32).reshape(nsel)
-                                          .contiguous(), torch.float32, (nsel,), "scales")
+    sc = None if scales is None else _flat(_on(solver, scales), nsel)
     if mode == 2:
         force, torque = solver.solid_loads_all, None
     else:

@@ -729,6 +729,9 @@ class PlainDomain:
         self.pos_dev = torch.zeros((S, 1, SEGMENTS, 3), dtype=torch.float32, device=dev)
         self.quat_dev = torch.zeros((S, 1, SEGMENTS, 4), dtype=torch.float32, device=dev)
         self.loads_dev = torch.zeros((req.substeps, SEGMENTS, 6), dtype=torch.float32, device=dev)
+        # each substep's rows: slicing them anew costs more host time than the copies themselves
+        self.rows = [(self.pos_dev[k], self.quat_dev[k], self.loads_dev[k, :, :3], self.loads_dev[k, :, 3:])
+                     for k in range(S)]
 
     def control_step(self) -> None:
         from . import coupling
@@ -740,12 +743,10 @@ class PlainDomain:
         self.quat_host.numpy()[:, 0] = quat
         self.pos_dev.copy_(self.pos_host, non_blocking=True)
         self.quat_dev.copy_(self.quat_host, non_blocking=True)
-        f = s.flows[0]
-        for k in range(S):
-            coupling.convert_and_update_solid_batch_3d(s, self.ids, self.pos_dev[k], self.quat_dev[k], self.zeros3,
-                                                       self.zeros3, self.ones)
+        for pos_k, quat_k, force_k, torque_k in self.rows:
+            coupling.convert_and_update_solid_batch_3d(s, self.ids, pos_k, quat_k, self.zeros3, self.zeros3, self.ones)
             s.step()
-            self.loads_dev[k, :, :3].copy_(f.solid_force)
-            self.loads_dev[k, :, 3:].copy_(f.solid_torque)
+            force_k.copy_(s.solid_force_all[0])
+            torque_k.copy_(s.solid_torque_all[0])
         self.loads.append(self.loads_dev.cpu().numpy())
         self.done += 1

@@ -87,3 +87,41 @@ def test_cut_links_of_few_and_many_segments(n_solids, n_seg, radius):
         got = np.stack([f.solid_forcex.cpu().numpy(), f.solid_forcey.cpu().numpy()], 1)
         assert np.abs(got).max() > 0
         assert np.abs(got - loads[:, :2]).max() <= 600 * 200 * eps
+
+
+def test_parameters_changed_in_place_reach_the_next_step():
+    """Viscosity, a boundary type or value, the body-force switch and an outline changed between
+    steps, in place or by assignment: the same bits as when the parameters are packed on every step."""
+    from openhomelbm_b200.lbm import LBM_Solver
+
+    def changes(s):
+        f = s.flows[1]
+        yield lambda: setattr(f, "vis_shear", 0.05)
+        yield lambda: f.bc_value.__setitem__((0, 0), 0.05)
+        yield lambda: f.bc_type.__setitem__(3, 0)
+        yield lambda: setattr(f, "bc_type", (0, 0, 1, 1))
+        yield lambda: setattr(f, "bc_value", [[0.02, 0.01], [0, 0], [0, 0], [0, 0]])
+        yield lambda: (f.force.fill_(1e-4), setattr(f, "use_force", True))
+        yield lambda: f.configure_solid(0, [(0.3, 0.0), (0.0, 0.3), (-0.3, 0.0), (0.0, -0.3)], (20.0, 15.0), scale=0.2)
+        yield lambda: setattr(f, "solid_line", f.solid_line.clone().mul_(0.5))
+
+    out = []
+    for always in (False, True):
+        s = LBM_Solver(48, 32, solid_num=1, nworld=2)
+        s.create_solid_from_polygon(0, [(0.2, 0.0), (0.0, 0.2), (-0.2, 0.0), (0.0, -0.2)], (24.0, 16.0), 0.2)
+        s.flows[1].bc_type = [0, 1, 1, 1]
+        seen = []
+        for change in changes(s):
+            change()
+            for _ in range(2):
+                if always:
+                    s._desc_key = None
+                s.step()
+            seen.append([f.cur.clone() for f in s.flows])
+        out.append(seen)
+    torch.cuda.synchronize()
+    for k, (a, b) in enumerate(zip(*out)):
+        for x, y in zip(a, b):
+            assert torch.equal(x, y), k
+        if k:
+            assert not torch.equal(a[1], out[0][k - 1][1]), k

@@ -404,7 +404,8 @@ __global__ void __launch_bounds__(TILE_THREADS) stream_tiles_kernel(const __grid
 }
 
 // ------------------------------------------------------------- 2c. stream over strips (a warp each)
-// Strip tiles of the work list: TX planes along x by STRIP_Y = 30 rows along y, one warp each.
+// Strips of a work list, or without one strips cut from a grid over the worlds (tiles == NULL, sx x sy of
+// them per world): TX planes along x by STRIP_Y = 30 rows along y, one warp each.
 // Lane l holds row y0 - 1 + l (lanes 0 and 31 are the strip's halo rows) and the warp marches its
 // source planes x0 - 1 .. x0 + TX. Each lane rebuilds its source cell's nine clamped populations
 // (feq_dev_clamped_a on its decoded moments, -w_i for a source outside a walled world: the same
@@ -422,16 +423,23 @@ constexpr int strip_min_blocks() { return TX == 32 && sizeof(typename S::T) <= 4
 
 template <class S, int TX>
 __global__ void __launch_bounds__(256, strip_min_blocks<S, TX>()) stream_strips_kernel(const __grid_constant__ Launch L,
-                                                            const int4* __restrict__ tiles, int n_tiles) {
+                                                            const int4* __restrict__ tiles, int n_tiles, int sx, int sy) {
   using R = typename S::R;
   using T = typename S::T;
   constexpr unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const int warps = gridDim.x * (blockDim.x >> 5);
   for (int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); t < n_tiles; t += warps) {
-    const int4 tile = tiles[t];
+    int4 tile;
+    if (tiles != nullptr) {
+      tile = tiles[t];
+    } else {  // strip t of sx x sy per world, x outer
+      const int w = t / (sx * sy), r = t - w * (sx * sy);
+      tile = make_int4(w, r / sy * TX, r % sy * STRIP_Y, 0);
+    }
     const World& wd = world_of(L, tile.x);
     const int nx = wd.nx, ny = wd.ny;
+    if (tile.y >= nx || tile.z >= ny) continue;  // past a world smaller than the largest
     const bool periodic = wd.periodic != 0;
     const float* __restrict__ fxp = wd.fx;
     const float* __restrict__ fyp = wd.fy;
@@ -444,7 +452,7 @@ __global__ void __launch_bounds__(256, strip_min_blocks<S, TX>()) stream_strips_
     const int x1 = x0 + TX < nx ? x0 + TX : nx;  // destination planes x0 .. x1 - 1
     const int yr = y0 - 1 + lane;                // this lane's row, before wrapping
     const int y = periodic ? wrap(yr, ny) : yr;
-    const bool y_in = periodic || (yr >= 0 && yr < ny);
+    const bool y_in = y >= 0 && y < ny;  // a world lower than a strip wraps once at most
     const bool dest_lane = lane >= 1 && lane <= STRIP_Y && yr < ny;
     // incoming populations of the last two source planes: c_x = 0 (i = 0, 3, 4) of the previous
     // plane, c_x = +1 (i = 1, 5, 8) of the previous two
@@ -1027,7 +1035,7 @@ template <class S, int TX> int launch_strips(const d2::Launch& L, const TileWork
   // ctas blocks of 8 warps, a warp per strip, no more blocks than the strips fill
   const int need = (tw.n_tiles + 7) / 8;
   const int grid = need < tw.ctas ? need : tw.ctas;
-  d2::stream_strips_kernel<S, TX><<<grid, 256, 0, st>>>(L, tw.tiles, tw.n_tiles);
+  d2::stream_strips_kernel<S, TX><<<grid, 256, 0, st>>>(L, tw.tiles, tw.n_tiles, 0, 0);
   HL_LAUNCH_CHECK("d2q9 stream_and_collide (strip work-list)");
   return HL_OK;
 }
@@ -1050,6 +1058,37 @@ template <class S> int stream_tiles(const d2::Launch& L, const TileWork& tw, cud
   return HL_ERR_ARG;
 }
 
+template <class S, int TX> int grid_strips(const d2::Launch& L, long long total, int sx, int sy, cudaStream_t st) {
+  d2::stream_strips_kernel<S, TX><<<unsigned((total + 3) / 4), 128, 0, st>>>(L, nullptr, int(total), sx, sy);
+  HL_LAUNCH_CHECK("d2q9 stream_and_collide (strips)");
+  return HL_OK;
+}
+
+// The stream phase without a work list: strips where they give every SM about 15 warps, the longest
+// that do (a strip of TX planes reads TX + 2); else a thread per cell, which rebuilds nine sources for
+// each cell but has more warps for a small launch. us, a thread per cell / strips of 4, 8, 16, 32:
+//   8 worlds 128 x 96 binary32      5.3 /   6.0   8.1  13.3  23.5
+//   12 of 203 x 117                10.2 /   7.6   9.7  14.6  24.6
+//   24 of 203 x 117                17.2 /  13.0  12.0  16.2  26.7
+//   64 of 256 x 200                90.6 /  86.1  73.7  64.6  52.8    binary16  105.8 / 75.3 65.3 55.1 58.6
+//   4096 x 2048                     206 /   204   169   152   112
+//   2048 x 2048 binary64            151 /   132   116   109   105
+template <class S> int stream_grid(const d2::Launch& L, int n, int maxx, int maxy, cudaStream_t st) {
+  const int sy = (maxy + d2::STRIP_Y - 1) / d2::STRIP_Y;
+  const long long least = 15ll * device_sms();
+  auto strips = [&](int tx) { return (long long)n * sy * ((maxx + tx - 1) / tx); };
+  if (strips(4) < least || strips(4) > 0x7fffffffll) {
+    dim3 grid((maxy + 31) / 32, (maxx + 7) / 8, n);
+    d2::stream_kernel<S><<<grid, 256, 0, st>>>(L);
+    HL_LAUNCH_CHECK("d2q9 stream_and_collide");
+    return HL_OK;
+  }
+  if (strips(32) >= least) return grid_strips<S, 32>(L, strips(32), (maxx + 31) / 32, sy, st);
+  if (strips(16) >= least) return grid_strips<S, 16>(L, strips(16), (maxx + 15) / 16, sy, st);
+  if (strips(8) >= least) return grid_strips<S, 8>(L, strips(8), (maxx + 7) / 8, sy, st);
+  return grid_strips<S, 4>(L, strips(4), (maxx + 3) / 4, sy, st);
+}
+
 template <class S> int run_phases(const d2::Launch& L, int n, int maxx, int maxy, bool any_solid, int phases,
                                   cudaStream_t st, const TileWork* tw = nullptr) {
   if ((phases & HL_PHASE_SEGMENTS) && any_solid) {
@@ -1061,9 +1100,8 @@ template <class S> int run_phases(const d2::Launch& L, int n, int maxx, int maxy
       const int rc = stream_tiles<S>(L, *tw, st);
       if (rc != HL_OK) return rc;
     } else {
-      dim3 grid((maxy + 31) / 32, (maxx + 7) / 8, n);
-      d2::stream_kernel<S><<<grid, 256, 0, st>>>(L);
-      HL_LAUNCH_CHECK("d2q9 stream_and_collide");
+      const int rc = stream_grid<S>(L, n, maxx, maxy, st);
+      if (rc != HL_OK) return rc;
     }
     if (any_solid) {
       d2::band_kernel<S><<<dim3(d2::BAND_BLOCKS, n), d2::BAND_THREADS, 0, st>>>(L);

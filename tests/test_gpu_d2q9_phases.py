@@ -125,3 +125,47 @@ def test_parameters_changed_in_place_reach_the_next_step():
             assert torch.equal(x, y), k
         if k:
             assert not torch.equal(a[1], out[0][k - 1][1]), k
+
+
+@pytest.mark.parametrize("storage", ["float32", "float16", "float64"])
+@pytest.mark.parametrize("nworld,nx,ny", [(1, 1501, 179), (1, 1499, 401), (1, 2003, 631), (1, 2111, 1097), (90, 61, 47),
+                                          (600, 33, 31), (1, 9001, 7)])
+def test_stream_without_a_work_list_equals_the_tiles(nworld, nx, ny, storage):
+    """The stream phase over a grid (a thread per cell, or strips of 4 to 32 planes by size) stores the
+    bits of the 8 x 32 tiles: walled worlds with solid cells inside and a body force, and periodic ones."""
+    from openhomelbm_b200 import _lib
+    from openhomelbm_b200.batching import TileConfig, WorldBatch2D
+    from openhomelbm_b200.lbm import LBM_Solver
+
+    torch.manual_seed(5)
+    for periodic in (False, True):
+        s = LBM_Solver(nx, ny, solid_num=1, nworld=nworld, storage=storage, periodic=periodic, u_scale=0.05, s_scale=2.5e-3)
+        for f in s.flows[:3] + s.flows[-1:]:
+            m = torch.rand((6, nx, ny), device="cuda", dtype=torch.float64) - 0.5
+            m[0] *= 0.1
+            if f.encoded:
+                f.moments[0].copy_(m)
+            else:
+                m[1:3] *= 0.1
+                m[3:] *= 0.02
+                f.moments[0].copy_(m)
+                f.moments[0][0] += 1.0
+            if not periodic:
+                f.flag[nx // 2 : nx // 2 + 3, ny // 3 : ny // 3 + 2] = 1
+                f.force.uniform_(-1e-4, 1e-4)
+                f.use_force = True
+        s._upload_descriptors()
+        st = _lib.stream_ptr()
+        _lib.check(_lib.lib().hl_d2q9_step_batch(_lib.ptr(s._desc_dev), nworld, 0, s.flows[0].storage_code, nx, ny, 0, 2, st))
+        got = [f.moments[1].clone() for f in s.flows]
+        for f in s.flows:
+            f.moments[1].zero_()
+            f.moments[1][0] = 0.0 if f.encoded else 1.0
+        b = WorldBatch2D(s.flows)
+        b.launch(0, st, TileConfig(8, 32, 1184), phases=2, any_solid=False)
+        torch.cuda.synchronize()
+        for k, f in enumerate(s.flows):
+            inner = got[k] if periodic else got[k][:, 1:-1, 1:-1]
+            want = f.moments[1] if periodic else f.moments[1][:, 1:-1, 1:-1]
+            assert torch.equal(inner, want), (periodic, k)
+        assert got[0].double().std() > 0

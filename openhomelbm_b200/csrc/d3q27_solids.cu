@@ -35,8 +35,8 @@
 // (1997), double-sided; a link is cut at the closest hit with 0 <= t <= 1 (the reference's
 // mesh query returns the closest hit up to max_t = 2, lbm_func_3d.py:308, and keeps it when
 // t <= 1). The triangles tested are those the solid's bin lists for the cell (all of them
-// without bins), screened by the warp against the box the cell's links reach, then paired
-// with the directions whose link segment box they meet; each pair is tested by one lane.
+// without bins), screened by the warp against the box the cell's links reach, then paired with
+// the directions whose link their box along the lattice's axes meets; each pair is tested by one lane.
 // The screens only drop triangles that cannot be hit with 0 <= t <= 1, so the hits are those
 // of a test against every triangle.
 
@@ -186,11 +186,6 @@ template <class R> __device__ __forceinline__ R warp_sum(R v) {
   return v;
 }
 template <class R> __device__ __forceinline__ R lane0(R v) { return __shfl_sync(0xffffffffu, v, 0); }
-__device__ __forceinline__ float warp_max(float v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-  return v;
-}
 
 // One near cell with a possible cut link, computed by a whole warp: lane i < 27 rebuilds the
 // population of direction i (a wall population with its momentum exchange if the link is
@@ -199,18 +194,35 @@ __device__ __forceinline__ float warp_max(float v) {
 constexpr unsigned FULL = 0xffffffffu;
 constexpr unsigned NO_HIT = 0xffffffffu;
 
-// Per-warp shared scratch of cut_cell, for the solid being tested: per direction its link's
-// segment box in the body frame (min xyz, pad, max xyz, pad; empty for an inactive
-// direction) and ray direction, the current chunk's triangles (slot = lane), the queue of
-// (direction, slot) pairs to test exactly, and per direction the bits of its closest hit.
+// Per-warp shared scratch of cut_cell, for the solid being tested: per direction its ray direction in
+// the body frame, the current chunk's triangles (slot = lane), the queue of (direction, slot) pairs to
+// test exactly, and per direction the bits of its closest hit.
 struct __align__(16) WarpScratch {
-  float seg[27 * 8];  // read as float4: 16-byte aligned at offset 0 of a 16-byte aligned struct
   float dir[27 * 3];
   float tri[32 * 9];
   unsigned q[32 * 27];
   unsigned best[32];
 };
-static_assert(sizeof(WarpScratch) % 16 == 0 && alignof(WarpScratch) == 16, "float4 reads of WarpScratch::seg");
+// The directions whose component along axis ax is v, as a bit mask.
+__host__ __device__ constexpr unsigned dir_mask(int ax, int v) {
+  constexpr signed char c[3][27] = {
+      {0, 1, -1, 0, 0, 0, 0, 1, -1, 1, -1, 0, 0, 1, -1, 1, -1, 0, 0, 1, -1, 1, -1, 1, -1, -1, 1},
+      {0, 0, 0, 1, -1, 0, 0, 1, -1, 0, 0, 1, -1, -1, 1, 0, 0, 1, -1, 1, -1, 1, -1, -1, 1, 1, -1},
+      {0, 0, 0, 0, 0, 1, -1, 0, 0, 1, -1, 1, -1, 0, 0, -1, 1, -1, 1, 1, -1, -1, 1, 1, -1, 1, -1}};
+  unsigned m = 0u;
+  for (int i = 0; i < 27; ++i) m |= c[ax][i] == v ? 1u << i : 0u;
+  return m;
+}
+// The directions whose link (0 to -c along axis ax, widened by e) the interval [lo, hi] meets. Not
+// dropped where a bound is NaN.
+template <int AX> __device__ __forceinline__ unsigned axis_dirs(float lo, float hi, float e) {
+  constexpr unsigned plus = dir_mask(AX, 1), zero = dir_mask(AX, 0), minus = dir_mask(AX, -1);
+  unsigned m = 0u;
+  if (!(lo > e || hi < -1.f - e)) m |= plus;
+  if (!(lo > e || hi < -e)) m |= zero;
+  if (!(lo > 1.f + e || hi < -e)) m |= minus;
+  return m;
+}
 
 template <class S>
 __device__ void cut_cell(const Args& a, double* acc, WarpScratch& ws, int x, int y, int z, unsigned mask) {
@@ -233,19 +245,22 @@ __device__ void cut_cell(const Args& a, double* acc, WarpScratch& ws, int x, int
   const bool active = i < 27 && xn >= 0 && xn < nx && yn >= 0 && yn < ny && zn >= 0 && zn < nz;
   // get_cutcell_multi_3d: the closest hit in [0, 1] over the solids near the cell. Which
   // solids and which candidate triangles depend on the cell only, so the loop is uniform
-  // across the warp. The warp screens the candidates 32 at a time (a lane per triangle)
-  // against the box that every link of the cell stays in, the cell's body-frame point
-  // +- the largest |component| of the lanes' ray directions, widened by 2e-3. That box holds
-  // each lane's segment box (widened by 1e-3), so a triangle outside it fails every lane's
-  // segment test: dropping it changes no hit. A survivor is tested exactly only for the
-  // directions whose segment box its bounding box meets (about a tenth of them): those
-  // (direction, triangle) pairs are queued and tested a pair per lane.
+  // across the warp. The warp screens the candidates 32 at a time (a lane per triangle) against the
+  // box that every link of the cell stays in, the cell's body-frame point +- the axes' images
+  // summed by magnitude, widened by 2e-3. A survivor's vertices are then taken to the lattice's axes
+  // with the cell as origin, where a link runs from 0 to -c: per axis its interval meets the links of
+  // some of c = -1, 0, 1 (widened by 1e-3 and by the rounding of the change of frame), and three
+  // masks of directions, one per axis, leave those that it can cut (27 box tests in the body frame
+  // took 36 and 45 us a launch at 64^3 and 160^3 with five 360-triangle bodies, this
+  // form 31 and 42). Those (direction, triangle) pairs are queued and tested a pair per lane.
   float cut = -1.f;  // geometry in binary32 (see the file comment)
   int sid = -1;
   const V3<R> cell{R(x), R(y), R(z)};
   const V3<R> dir{-dx, -dy, -dz};
   const V3<float> gcell{float(x), float(y), float(z)};
   const V3<float> gdir{-float(ix), -float(iy), -float(iz)};
+  // the rest direction's link has no length: no triangle is hit along it
+  const unsigned tested = __ballot_sync(FULL, active) & ~1u;
   for (int k = 0; k < s.n_objects; ++k) {
     if (!in_mask(mask, k)) continue;  // no candidate triangles for this cell's rays
     const int t0 = s.tri_offset[k], ntri = s.tri_offset[k + 1] - t0;
@@ -262,25 +277,28 @@ __device__ void cut_cell(const Args& a, double* acc, WarpScratch& ws, int x, int
     const int32_t* list;
     int ncand;
     if (!candidates(s, k, ntri, los, sx, sy, sz, &list, &ncand)) continue;
-    const float rx = warp_max(i < 27 ? float(fabs(lds.x)) : 0.f) + 2e-3f;
-    const float ry = warp_max(i < 27 ? float(fabs(lds.y)) : 0.f) + 2e-3f;
-    const float rz = warp_max(i < 27 ? float(fabs(lds.z)) : 0.f) + 2e-3f;
+    // the images of the lattice's axes in the body frame (directions 1, 3 and 5 run along them) and
+    // the inverse map's rows, whatever the transform's rotation and scale are
+    const V3<float> ax{-__shfl_sync(FULL, lds.x, 1), -__shfl_sync(FULL, lds.y, 1), -__shfl_sync(FULL, lds.z, 1)};
+    const V3<float> ay{-__shfl_sync(FULL, lds.x, 3), -__shfl_sync(FULL, lds.y, 3), -__shfl_sync(FULL, lds.z, 3)};
+    const V3<float> az{-__shfl_sync(FULL, lds.x, 5), -__shfl_sync(FULL, lds.y, 5), -__shfl_sync(FULL, lds.z, 5)};
+    V3<float> wx{ay.y * az.z - ay.z * az.y, ay.z * az.x - ay.x * az.z, ay.x * az.y - ay.y * az.x};
+    V3<float> wy{az.y * ax.z - az.z * ax.y, az.z * ax.x - az.x * ax.z, az.x * ax.y - az.y * ax.x};
+    V3<float> wz{ax.y * ay.z - ax.z * ay.y, ax.z * ay.x - ax.x * ay.z, ax.x * ay.y - ax.y * ay.x};
+    const float det = ax.x * wx.x + ax.y * wx.y + ax.z * wx.z;
+    const bool invertible = fabsf(det) > 1e-30f;
+    const float inv_det = 1.f / det;
+    wx = {wx.x * inv_det, wx.y * inv_det, wx.z * inv_det};
+    wy = {wy.x * inv_det, wy.y * inv_det, wy.z * inv_det};
+    wz = {wz.x * inv_det, wz.y * inv_det, wz.z * inv_det};
+    const float rx = (fabsf(ax.x) + fabsf(ay.x) + fabsf(az.x)) * 1.000001f + 2e-3f;
+    const float ry = (fabsf(ax.y) + fabsf(ay.y) + fabsf(az.y)) * 1.000001f + 2e-3f;
+    const float rz = (fabsf(ax.z) + fabsf(ay.z) + fabsf(az.z)) * 1.000001f + 2e-3f;
     const float bx0 = float(los.x) - rx, bx1 = float(los.x) + rx;
     const float by0 = float(los.y) - ry, by1 = float(los.y) + ry;
     const float bz0 = float(los.z) - rz, bz1 = float(los.z) + rz;
     const float* tk = s.tris + 9ll * t0;
-    // this solid's segment boxes and ray directions, one direction per lane
-    const float eps = 1e-3f, inf = __int_as_float(0x7f800000);
-    if (i < 27) {
-      float* sb = ws.seg + 8 * i;
-      sb[0] = active ? fminf(los.x, los.x + lds.x) - eps : inf;
-      sb[1] = active ? fminf(los.y, los.y + lds.y) - eps : inf;
-      sb[2] = active ? fminf(los.z, los.z + lds.z) - eps : inf;
-      sb[4] = active ? fmaxf(los.x, los.x + lds.x) + eps : -inf;
-      sb[5] = active ? fmaxf(los.y, los.y + lds.y) + eps : -inf;
-      sb[6] = active ? fmaxf(los.z, los.z + lds.z) + eps : -inf;
-      ws.dir[3 * i] = lds.x, ws.dir[3 * i + 1] = lds.y, ws.dir[3 * i + 2] = lds.z;
-    }
+    if (i < 27) ws.dir[3 * i] = lds.x, ws.dir[3 * i + 1] = lds.y, ws.dir[3 * i + 2] = lds.z;
     ws.best[i] = NO_HIT;
     __syncwarp();
     // software pipeline over the chunks: the vertices of chunk q + 1 and the list entries of
@@ -308,15 +326,24 @@ __device__ void cut_cell(const Args& a, double* acc, WarpScratch& ws, int x, int
       const float mnz = fminf(fminf(v[2], v[5]), v[8]), mxz = fmaxf(fmaxf(v[2], v[5]), v[8]);
       const bool keep = live && !(mxx < bx0 || mnx > bx1 || mxy < by0 || mny > by1 || mxz < bz0 || mnz > bz1);
       if (__ballot_sync(FULL, keep) == 0u) continue;  // uniform
-      // the directions whose segment box this lane's triangle meets (27 independent tests)
+      // the directions whose link this lane's triangle can cut
       unsigned dm = 0u;
       if (keep) {
-#pragma unroll 9
-        for (int d = 0; d < 27; ++d) {
-          const float4 l4 = *reinterpret_cast<const float4*>(ws.seg + 8 * d);
-          const float4 h4 = *reinterpret_cast<const float4*>(ws.seg + 8 * d + 4);
-          if (!(mxx < l4.x || mnx > h4.x || mxy < l4.y || mny > h4.y || mxz < l4.z || mnz > h4.z)) dm |= 1u << d;
+        float lx[3], ly[3], lz[3];
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+          const float px = v[3 * j] - los.x, py = v[3 * j + 1] - los.y, pz = v[3 * j + 2] - los.z;
+          lx[j] = fmaf(wx.x, px, fmaf(wx.y, py, wx.z * pz));
+          ly[j] = fmaf(wy.x, px, fmaf(wy.y, py, wy.z * pz));
+          lz[j] = fmaf(wz.x, px, fmaf(wz.y, py, wz.z * pz));
         }
+        const float x0 = fminf(fminf(lx[0], lx[1]), lx[2]), x1 = fmaxf(fmaxf(lx[0], lx[1]), lx[2]);
+        const float y0 = fminf(fminf(ly[0], ly[1]), ly[2]), y1 = fmaxf(fmaxf(ly[0], ly[1]), ly[2]);
+        const float z0 = fminf(fminf(lz[0], lz[1]), lz[2]), z1 = fmaxf(fmaxf(lz[0], lz[1]), lz[2]);
+        const float far = fmaxf(fmaxf(fmaxf(-x0, x1), fmaxf(-y0, y1)), fmaxf(-z0, z1));
+        const float e = fmaf(4e-6f, far, 1e-3f);
+        dm = tested;
+        if (invertible) dm &= axis_dirs<0>(x0, x1, e) & axis_dirs<1>(y0, y1, e) & axis_dirs<2>(z0, z1, e);
         if (dm) {
 #pragma unroll
           for (int j = 0; j < 9; ++j) ws.tri[9 * i + j] = v[j];
@@ -418,11 +445,13 @@ __device__ void cut_cell(const Args& a, double* acc, WarpScratch& ws, int x, int
   for (unsigned left = __ballot_sync(0xffffffffu, pend >= 0); left; left = __ballot_sync(0xffffffffu, pend >= 0)) {
     const int target = __shfl_sync(0xffffffffu, pend, __ffs(left) - 1);
     const bool mine = pend == target;
+    double sum = 0.0;  // lane j < 6 adds component j, six at once
 #pragma unroll
     for (int j = 0; j < 6; ++j) {
       const double v = warp_sum(mine ? lf[j] : 0.0);
-      if (i == 0) atomicAdd(&acc[6 * target + j], v);
+      if (i == j) sum = v;
     }
+    if (i < 6) atomicAdd(&acc[6 * target + i], sum);
     if (mine) pend = -1;
   }
   // moments (lbm_func_3d.py:528-562) as warp sums: rho, the signed first moments and the
@@ -591,10 +620,12 @@ __device__ __forceinline__ void loads_out(const hl_solids3d& s, int k) {
 }
 
 // The block that finishes last (work[1] counts finished blocks) writes the binary32 loads.
-// Blocks of 16 warps (one per SM at 104 registers), each warp's scratch in dynamic shared
+// Blocks of 20 warps (one per SM at 96 registers), each warp's scratch in dynamic shared
 // memory: a warp spends most of a cell waiting on dependent loads, so more warps per SM hide
-// more of it than the same warps spread over more SMs.
-constexpr int PBLOCK = 512;
+// more of it than the same warps spread over more SMs. Warps a block 16 / 20 / 24 / 32, us: eight
+// substeps of a 160^3 swimmer 1515 / 1498 / 1503 / 1511, of a 64^3 one 638 / 640 / 648 / 678, of nine
+// served domains 5680 / 5557 / 5510 / 5548.
+constexpr int PBLOCK = 640;
 constexpr int PBLOCK_SMEM = int(sizeof(WarpScratch)) * (PBLOCK / 32);
 template <class S> __global__ void __launch_bounds__(PBLOCK) process_kernel(const __grid_constant__ Args a) {
   __shared__ double acc[MAX_SOLIDS * 6];
@@ -735,7 +766,7 @@ template <class S> int launch(const hl_world3d* w, double vis, const hl_solids3d
     if (e != cudaSuccess) return cuda_status(e, "d3q27 solid links: zero work count");
     classify_kernel<S><<<grid, BLOCK, 0, st>>>(a);
     HL_LAUNCH_CHECK("d3q27 solid links (classify)");
-    // one 16-warp block per SM unless set; the last block to finish writes the binary32 loads
+    // one block per SM unless set; the last block to finish writes the binary32 loads
     const int blocks = g_tune_d3_link_blocks > 0 ? g_tune_d3_link_blocks : num_sms_local();
     const int ar = set_smem_attr(reinterpret_cast<const void*>(&process_kernel<S>), PBLOCK_SMEM,
                                  "d3q27 solid links (cut cells)");

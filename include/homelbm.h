@@ -183,9 +183,9 @@ HL_API int hl_d3q27_stream_collide_batch(const void* desc, int n_domains, int n_
 HL_API size_t hl_d3q27_bc_scratch_bytes(const hl_world3d* w);
 
 /* Batched boundaries (the serving form's batched substep; no reference counterpart: the
- * reference runs apply_bc_3d per world, envs/lbm3d/lbm_solver_3d.py:88-127). The three waves
- * of hl_d3q27_apply_bc run as three launches over all domains of a set instead of three per
- * domain; per cell the same result as hl_d3q27_apply_bc on each domain.
+ * reference runs apply_bc_3d per world, envs/lbm3d/lbm_solver_3d.py:88-127): one launch (or
+ * three, where a world has a side of three cells) over all domains of a set instead of as many
+ * per domain; per cell the same result as hl_d3q27_apply_bc on each domain.
  *  - hl_d3q27_bc_batch_bytes: device bytes of the descriptors of n domains.
  *  - hl_d3q27_bc_batch_prepare: writes the descriptors of worlds[0 .. n) (given at parity 0:
  *    the step reads cur and writes post), their conditions bcs[i] and boundary scratch

@@ -12,6 +12,7 @@
 //                 binary32 copies of the loads (solid_forcex, solid_forcey, torque).
 // Cells in the band are computed twice; the band is a small part of the domain.
 
+#include <algorithm>
 #include <cmath>
 
 #include "hl_common.cuh"
@@ -608,9 +609,9 @@ __device__ __forceinline__ Cut get_cutcell_list(const World& w, const float4* se
 }
 
 constexpr int BAND_SEGS = 1024;       // segments staged per block
-constexpr int BAND_THREADS = 128;     // cells of a block's pass
+constexpr int BAND_CELLS = 128;       // cells of a block's pass
 constexpr int BAND_CAND = 16;         // candidate segments kept per cell; more: the full scan
-constexpr int BAND_BLOCKS = 96;       // blocks per world
+constexpr int BAND_BLOCKS = 96;       // blocks per world, fewer where many worlds share the chip
 
 // The cells near a solid. Only a few cells of a block lie next to an outline, and a cut cell is nine
 // links, each a search and a load, so a block takes its cells in three passes: a thread per outline
@@ -618,8 +619,8 @@ constexpr int BAND_BLOCKS = 96;       // blocks per world
 // was most of the time); the threads then take the noted cells' links, one (cell, link) each; and a
 // thread per cut cell collides its nine populations. A thread per cell through all of it had 9
 // threads of a warp active: 35 us for one 96-sided outline at 512 x 128 and 98 us for 60 worlds of
-// eight 26-sided ones; this form takes 13.6 and 64.
-template <class S> __global__ void __launch_bounds__(BAND_THREADS) band_kernel(const __grid_constant__ Launch L) {
+// eight 26-sided ones; this form takes 9.9 and 56.
+template <class S, int THREADS> __global__ void __launch_bounds__(THREADS) band_kernel(const __grid_constant__ Launch L) {
   using R = typename S::R;
   using T = typename S::T;
   constexpr unsigned FULL = 0xffffffffu;
@@ -630,22 +631,22 @@ template <class S> __global__ void __launch_bounds__(BAND_THREADS) band_kernel(c
   const int bw = y1 - y0 + 1;
   const long long area = (long long)(x1 - x0 + 1) * bw;
   // (block-uniform) a block past the end of the band has no cell
-  if (x0 > x1 || y0 > y1 || (long long)blockIdx.x * BAND_THREADS >= area) return;
+  if (x0 > x1 || y0 > y1 || (long long)blockIdx.x * BAND_CELLS >= area) return;
   __shared__ double acc[MAX_SOLIDS * 3];
   // the world's per-solid band radii and segments, read by every cell's screening and ray
   // tests: staged in shared memory (the segments when they fit)
   __shared__ float4 s_seg[BAND_SEGS];
   __shared__ float s_px[MAX_SOLIDS], s_py[MAX_SOLIDS], s_r2[MAX_SOLIDS];
   __shared__ int s_nseg[MAX_SOLIDS];
-  __shared__ R s_pop[BAND_THREADS * 9];
-  __shared__ int s_cell[BAND_THREADS], s_count[BAND_THREADS], s_cut[BAND_THREADS];
-  __shared__ int s_cand[BAND_THREADS * BAND_CAND];
+  __shared__ R s_pop[BAND_CELLS * 9];
+  __shared__ int s_cell[BAND_CELLS], s_count[BAND_CELLS], s_cut[BAND_CELLS];
+  __shared__ int s_cand[BAND_CELLS * BAND_CAND];
   __shared__ int n_listed, touched;
   const int nsol = min(w.n_objects, MAX_SOLIDS);
   const int max_seg = w.max_segments, n_seg = w.n_objects * max_seg;
   const float4* segs = n_seg <= BAND_SEGS ? s_seg : nullptr;
-  for (int k = tid; k < nsol * 3; k += BAND_THREADS) acc[k] = 0.0;
-  for (int s = tid; s < nsol; s += BAND_THREADS) {
+  for (int k = tid; k < nsol * 3; k += THREADS) acc[k] = 0.0;
+  for (int s = tid; s < nsol; s += THREADS) {
     const float scale = w.scale[s] * float(w.nx);
     s_px[s] = w.position[2 * s];
     s_py[s] = w.position[2 * s + 1];
@@ -653,21 +654,21 @@ template <class S> __global__ void __launch_bounds__(BAND_THREADS) band_kernel(c
     s_nseg[s] = w.line_num[s];
   }
   if (segs)
-    for (int j = tid; j < n_seg; j += BAND_THREADS) s_seg[j] = segment_of(w, j);
+    for (int j = tid; j < n_seg; j += THREADS) s_seg[j] = segment_of(w, j);
   if (tid == 0) n_listed = touched = 0;
-  s_count[tid] = 0;
+  if (tid < BAND_CELLS) s_count[tid] = 0;
   __syncthreads();
   const long long N = (long long)w.nx * w.ny;
   const T* cur = static_cast<const T*>(cur_of(L, w));
-  for (long long k0 = (long long)blockIdx.x * BAND_THREADS; k0 < area; k0 += (long long)gridDim.x * BAND_THREADS) {
+  for (long long k0 = (long long)blockIdx.x * BAND_CELLS; k0 < area; k0 += (long long)gridDim.x * BAND_CELLS) {
     // 1. The segments of the near solids (get_cutcell's radius test) that can cross a link of a
     // cell: every link lies in the square [x-1, x+1] x [y-1, y+1], so a segment whose box misses that
     // square widened by 1e-3 crosses none. No candidate: no cut link, and the stream kernel's value
     // is already the cell's update. The pass's cells are rows xa .. xb of the box, clipped.
-    const int k_end = int(area - k0 < BAND_THREADS ? area - k0 : BAND_THREADS);
+    const int k_end = int(area - k0 < BAND_CELLS ? area - k0 : BAND_CELLS);
     const int xa = x0 + int(k0 / bw), ya = y0 + int(k0 % bw);  // the pass's first and last cell
     const int xb = x0 + int((k0 + k_end - 1) / bw), yb = y0 + int((k0 + k_end - 1) % bw);
-    for (int j = tid; j < 4 * n_seg; j += BAND_THREADS) {  // four threads a segment, every fourth row each
+    for (int j = tid; j < 4 * n_seg; j += THREADS) {  // four threads a segment, every fourth row each
       const int id = j >> 2, s = id / max_seg;
       if (id - s * max_seg >= s_nseg[s]) continue;
       const float4 g = segs ? segs[id] : segment_of(w, id);
@@ -704,7 +705,7 @@ template <class S> __global__ void __launch_bounds__(BAND_THREADS) band_kernel(c
     __syncthreads();
     const int listed = n_listed;
     // 2. the links of the listed cells
-    for (int it0 = 0; it0 < listed * 9; it0 += BAND_THREADS) {
+    for (int it0 = 0; it0 < listed * 9; it0 += THREADS) {
       const int it = it0 + tid;
       int hit_solid = -1;
       double lf[3] = {0.0, 0.0, 0.0};
@@ -720,13 +721,15 @@ template <class S> __global__ void __launch_bounds__(BAND_THREADS) band_kernel(c
         }
         R pop = -w2<R>(i);
         if (xn >= 0 && xn < w.nx && yn >= 0 && yn < w.ny) {
-          const Mom2<R> mn = load2<S>(w, N, (long long)xn * w.ny + yn, cur);  // the upwind neighbour
+          // the upwind neighbour, and the cell itself for a cut link (loaded together: a chain of
+          // loads is what a link takes)
+          const Mom2<R> mn = load2<S>(w, N, (long long)xn * w.ny + yn, cur);
+          const Mom2<R> me = load2<S>(w, N, (long long)cx * w.ny + cy, cur);
           const int nc = s_count[at];
           const Cut cc = nc > BAND_CAND ? get_cutcell(w, float(cx), float(cy), float(dx), float(dy))
                                         : get_cutcell_list(w, segs, s_cand + at * BAND_CAND, nc, float(cx), float(cy),
                                                            float(dx), float(dy));
           if (cc.t >= 0.f && cc.solid >= 0) {
-            const Mom2<R> me = load2<S>(w, N, (long long)cx * w.ny + cy, cur);
             s_cut[at] = 1;
             const int s = cc.solid, nseg = s_nseg[s];
             const int n1 = cc.seg + 1 == nseg ? 0 : cc.seg + 1;
@@ -765,13 +768,15 @@ template <class S> __global__ void __launch_bounds__(BAND_THREADS) band_kernel(c
       for (unsigned left = __ballot_sync(FULL, hit_solid >= 0); left; left = __ballot_sync(FULL, hit_solid >= 0)) {
         const int target = __shfl_sync(FULL, hit_solid, __ffs(left) - 1);
         const bool mine = hit_solid == target;
+        double sum = 0.0;  // lane j < 3 adds component j, three at once
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
           double v = mine ? lf[j] : 0.0;
 #pragma unroll
           for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(FULL, v, o);
-          if (lane == 0) atomicAdd(&acc[3 * target + j], v);
+          if (lane == j) sum = v;
         }
+        if (lane < 3) atomicAdd(&acc[3 * target + lane], sum);
         if (lane == 0) touched = 1;
         if (mine) hit_solid = -1;
       }
@@ -789,11 +794,11 @@ template <class S> __global__ void __launch_bounds__(BAND_THREADS) band_kernel(c
     }
     __syncthreads();
     if (tid == 0) n_listed = 0;
-    s_count[tid] = 0;
+    if (tid < BAND_CELLS) s_count[tid] = 0;
     __syncthreads();
   }
   if (touched)
-    for (int k = tid; k < nsol * 3; k += BAND_THREADS)
+    for (int k = tid; k < nsol * 3; k += THREADS)
       if (acc[k] != 0.0) atomicAdd(&w.loads64[k], acc[k]);
 }
 
@@ -1104,7 +1109,17 @@ template <class S> int run_phases(const d2::Launch& L, int n, int maxx, int maxy
       if (rc != HL_OK) return rc;
     }
     if (any_solid) {
-      d2::band_kernel<S><<<dim3(d2::BAND_BLOCKS, n), d2::BAND_THREADS, 0, st>>>(L);
+      // A pass's links are a chain of loads and searches, so while all worlds' blocks are resident at
+      // once (about eight per SM) 256 threads take them in one go; more worlds fill the chip with 128
+      // threads and fewer blocks each, as most blocks of a small band only look at its box. us,
+      // 256 x 96 / 128 x 96 / 128 x 48 / 128 x 24, worlds of two 32-sided outlines at 203 x 117: one 9.4 /
+      // 11.8 / 11.8 / 17.3, eight 10.9 / 12.6 / 12.8 / 18.0, 12 13.1 / 13.9 / 13.2 / 18.5, 24 21.7 / 17.8 / 17.3 /
+      // 20.0, 48 37.3 / 28.3 / 26.6 / 25.7; 60 worlds of eight 26-sided ones 62.5 / 61.6 / 57.7 / 55.8.
+      const int per = 8 * device_sms() / n;
+      if (per >= d2::BAND_BLOCKS)
+        d2::band_kernel<S, 256><<<dim3(d2::BAND_BLOCKS, n), 256, 0, st>>>(L);
+      else
+        d2::band_kernel<S, 128><<<dim3(std::min(std::max(per, 24), 48), n), 128, 0, st>>>(L);
       HL_LAUNCH_CHECK("d2q9 cut-cell band");
     }
   }

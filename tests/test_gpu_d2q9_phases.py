@@ -169,3 +169,33 @@ def test_stream_without_a_work_list_equals_the_tiles(nworld, nx, ny, storage):
             want = f.moments[1] if periodic else f.moments[1][:, 1:-1, 1:-1]
             assert torch.equal(inner, want), (periodic, k)
         assert got[0].double().std() > 0
+
+
+@pytest.mark.parametrize("nworld", [11, 16, 49])
+def test_cut_links_of_many_worlds_equal_one(nworld):
+    """The cut links of a world among many (fewer, smaller blocks each) store the bits that it gets alone;
+    its loads are the same binary64 sums in another order, within 64 links * 2^-52 of their magnitude,
+    rounded to binary32 (2^-23)."""
+    from openhomelbm_b200.lbm import LBM_Solver
+
+    def run(n):
+        s = LBM_Solver(150, 97, solid_num=2, nworld=n)
+        m = torch.tensor(_state(150, 97, 3), device="cuda")
+        for f in s.flows:
+            for buf in f.moments:
+                buf.copy_(m)
+        ang = np.linspace(0, 2 * np.pi, 40, endpoint=False)
+        ring = [(0.5 * np.cos(a), 0.5 * np.sin(a)) for a in ang]
+        s.create_solid_from_polygon(0, ring, (50.3, 48.6), 0.3)
+        s.create_solid_from_polygon(1, ring, (100.2, 47.1), 0.2)
+        for _ in range(3):
+            s.step()
+        torch.cuda.synchronize()
+        return s
+
+    one, many = run(1), run(nworld)
+    loads = one.solid_loads_all[0].double()
+    assert loads.abs().max() > 0
+    for w, f in enumerate(many.flows):
+        assert torch.equal(f.cur, one.flows[0].cur), w
+        assert (many.solid_loads_all[w].double() - loads).abs().max() <= loads.abs().max() * 2.0 ** -22, w

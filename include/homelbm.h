@@ -62,7 +62,7 @@ HL_API const char* hl_version(void);
  *     hl_d3q27_stream_collide at launch and by hl_d3q27_batch_prepare)
  *   "d3q27_stages": 0, 3..5: accepted, without effect (the staging depth is fixed per storage type)
  *   "d3q27_link_blocks": 0 automatic, k > 0 blocks of the cut-link kernel over the listed
- *     cells (fewer leave SMs free for other domains' kernels on other streams): blocks of 16
+ *     cells (fewer leave SMs free for other domains' kernels on other streams): blocks of 20
  *     warps for hl_d3q27_solid_links (automatic: one per SM), of 4 warps for
  *     hl_d3q27_solid_links_batch (automatic: four per SM)
  * Returns HL_ERR_ARG for an unknown key. A CUDA graph keeps the choice it was captured with. */
@@ -148,8 +148,9 @@ HL_API size_t hl_d3q27_scratch_bytes(const hl_world3d* w);
  *  - Computes what hl_d3q27_stream_collide computes with a non-NULL diag: post <- step(cur),
  *    *mass (binary64 sum of rho over updated cells) and *health (count of updated cells with
  *    non-finite moments or rho <= 0); mass and health may be NULL. Storage float32 or
- *    float64 (other storages return HL_ERR_ARG); it always runs the general kernel, never
- *    the TMA-staged one, so its results can differ from hl_d3q27_stream_collide in rounding.
+ *    float64 (other storages return HL_ERR_ARG); it always runs the kernels that take rows of
+ *    any length, never a TMA-staged one, so its results can differ from hl_d3q27_stream_collide in
+ *    rounding.
  *  - Limit: 64 + 12 bytes for each of two CTAs per SM, i.e. devices with up to 680 SMs (a B200 has
  *    148); larger needs are rejected with HL_ERR_ARG.
  *  - The first call on a device resolves the array's device address (cudaGetSymbolAddress,

@@ -535,7 +535,7 @@ class ServeEngine:
             raise ValueError(f"x_chunks must be >= 0, got {x_chunks}")
         # blocks of each domain's cut-link kernel (the library's "d3q27_link_blocks" while run()
         # lasts; 0 keeps the library's automatic grid). None: a quarter of the SM count for
-        # per-domain graphs (16-warp blocks: 592 warps on a 148-SM B200), 0 for the batched form:
+        # per-domain graphs (20-warp blocks: 740 warps on a 148-SM B200), 0 for the batched form:
         # with resident domains sharing the GPU, fewer blocks per domain leave the other domains'
         # kernels room.
         if link_blocks is None:

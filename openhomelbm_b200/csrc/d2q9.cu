@@ -567,11 +567,13 @@ __device__ Cut get_cutcell(const World& w, float x, float y, float dx, float dy)
   return r;
 }
 
-// Segment j = solid * max_segments + n of a world: its end points (x, y) and (z, w).
+// Segment j = solid * max_segments + n of a world: its end points (x, y) and (z, w). A slot past the
+// outline's last segment (a solid may have fewer than max_segments, or none) gives a value that nobody
+// uses, read from the solid's own slots.
 __device__ __forceinline__ float4 segment_of(const World& w, int j) {
   const int s = j / w.max_segments, n = j - s * w.max_segments;
   const float* tf = w.tf + size_t(s) * w.max_segments * 2;
-  const int n1 = n + 1 == w.line_num[s] ? 0 : n + 1;
+  const int n1 = n + 1 < w.line_num[s] ? n + 1 : 0;
   return make_float4(tf[2 * n], tf[2 * n + 1], tf[2 * n1], tf[2 * n1 + 1]);
 }
 

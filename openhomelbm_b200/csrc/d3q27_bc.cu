@@ -79,26 +79,42 @@ template <class S> __device__ __forceinline__ void copy_raw(const BcArgs& a, lon
 #pragma unroll
   for (int k = 0; k < 10; ++k) dst[k] = p[k * a.N + i];
 }
-template <class S> __device__ __forceinline__ void encode_cell(const Mom3<typename S::R>& m, const Scale& sc, typename S::R raw[10]) {
+// One value of a boundary cell, whichever kernel computes it, has the same bits: a 16-bit storage draws
+// its rounding noise from them, so every product and sum below is fixed as fused or not. FACE: cells on one
+// face. The 16-bit storages' cells on two or three faces round their products the other way round; those
+// are the forms that stored fields have had from the first, and other ones would draw other noise.
+__device__ __forceinline__ float fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+// the equilibrium's stress difference between velocities a and b, one component
+template <class S, bool FACE, class R> __device__ __forceinline__ R feq_gap(R a1, R a2, R b1, R b2) {
+  if constexpr (S::kEncoded && !FACE) return fma_rn(-b1, b2, mul_rn(a1, a2));
+  else return fma_rn(a1, a2, -mul_rn(b1, b2));
+}
+template <class S, bool FACE>
+__device__ __forceinline__ void encode_cell(const Mom3<typename S::R>& m, const Scale& sc, typename S::R raw[10]) {
   if constexpr (S::kEncoded) {
+    auto n = [](float a, float b, float s) { return FACE ? fma_rn(-a, b, s) : __fsub_rn(s, mul_rn(a, b)); };
     raw[0] = m.drho;
     raw[1] = m.ux * sc.inv_u;
     raw[2] = m.uy * sc.inv_u;
     raw[3] = m.uz * sc.inv_u;
-    raw[4] = fmaf(-m.ux, m.ux, m.sxx) * sc.inv_s;
-    raw[5] = fmaf(-m.uy, m.uy, m.syy) * sc.inv_s;
-    raw[6] = fmaf(-m.uz, m.uz, m.szz) * sc.inv_s;
-    raw[7] = fmaf(-m.ux, m.uy, m.sxy) * sc.inv_s;
-    raw[8] = fmaf(-m.ux, m.uz, m.sxz) * sc.inv_s;
-    raw[9] = fmaf(-m.uy, m.uz, m.syz) * sc.inv_s;
+    raw[4] = n(m.ux, m.ux, m.sxx) * sc.inv_s;
+    raw[5] = n(m.uy, m.uy, m.syy) * sc.inv_s;
+    raw[6] = n(m.uz, m.uz, m.szz) * sc.inv_s;
+    raw[7] = n(m.ux, m.uy, m.sxy) * sc.inv_s;
+    raw[8] = n(m.ux, m.uz, m.sxz) * sc.inv_s;
+    raw[9] = n(m.uy, m.uz, m.syz) * sc.inv_s;
   } else {
     encode3<S>(m, sc, raw);
   }
 }
-template <class S> __device__ __forceinline__ void store_cell(const BcArgs& a, long long i, const Mom3<typename S::R>& m) {
+template <class S, bool FACE>
+__device__ __forceinline__ void store_cell(const BcArgs& a, long long i, const Mom3<typename S::R>& m) {
   typename S::T* p = static_cast<typename S::T*>(a.post);
   typename S::R raw[10];
-  encode_cell<S>(m, a.sc, raw);
+  encode_cell<S, FACE>(m, a.sc, raw);
 #pragma unroll
   for (int k = 0; k < 10; ++k) p[k * a.N + i] = S::from_r(raw[k], unsigned(k * a.N + i));
 }
@@ -110,18 +126,12 @@ template <class S> __device__ __forceinline__ void store_cell(const BcArgs& a, l
 // delta_ac delta_bd + delta_ad delta_bc) / 9, so P_ab = (rho - 1) delta_ab / 3 + rho u_a u_b
 // and S_ab = u_a u_b exactly: computed in that closed form, not as the reference's 27-term
 // binary32 sums (which agree with it to their rounding).
-// The products are fused explicitly, here and in encode_cell, so that every kernel that computes a
-// cell gets the same bits (16-bit storages draw their rounding noise from them).
-__device__ __forceinline__ float fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
-__device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
-__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
-__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
-// the equilibrium's stress difference between velocities a and b, one component
-template <class R> __device__ __forceinline__ R feq_gap(R a1, R a2, R b1, R b2) { return fma_rn(a1, a2, -mul_rn(b1, b2)); }
 
 // apply_bc_core_3d (envs/lbm3d/lbm_func_3d.py:627-648): new state of boundary cell t from
 // its own old state and its inward neighbour nb.
-template <class R> __device__ Mom3<R> bc_core(const BcArgs& a, int dr, const Mom3<R>& t, const Mom3<R>& nb) {
+template <class S, bool FACE>
+__device__ Mom3<typename S::R> bc_core(const BcArgs& a, int dr, const Mom3<typename S::R>& t, const Mom3<typename S::R>& nb) {
+  using R = typename S::R;
   Mom3<R> r = t;
   if (a.bc_type[dr] == 0) {
     r.ux = R(a.bc_value[dr][0]);
@@ -134,12 +144,12 @@ template <class R> __device__ Mom3<R> bc_core(const BcArgs& a, int dr, const Mom
   }
   r.rho = nb.rho;
   r.drho = nb.drho;
-  r.sxx = feq_gap(r.ux, r.ux, nb.ux, nb.ux) + nb.sxx;
-  r.syy = feq_gap(r.uy, r.uy, nb.uy, nb.uy) + nb.syy;
-  r.szz = feq_gap(r.uz, r.uz, nb.uz, nb.uz) + nb.szz;
-  r.sxy = feq_gap(r.ux, r.uy, nb.ux, nb.uy) + nb.sxy;
-  r.sxz = feq_gap(r.ux, r.uz, nb.ux, nb.uz) + nb.sxz;
-  r.syz = feq_gap(r.uy, r.uz, nb.uy, nb.uz) + nb.syz;
+  r.sxx = feq_gap<S, FACE>(r.ux, r.ux, nb.ux, nb.ux) + nb.sxx;
+  r.syy = feq_gap<S, FACE>(r.uy, r.uy, nb.uy, nb.uy) + nb.syy;
+  r.szz = feq_gap<S, FACE>(r.uz, r.uz, nb.uz, nb.uz) + nb.szz;
+  r.sxy = feq_gap<S, FACE>(r.ux, r.uy, nb.ux, nb.uy) + nb.sxy;
+  r.sxz = feq_gap<S, FACE>(r.ux, r.uz, nb.ux, nb.uz) + nb.sxz;
+  r.syz = feq_gap<S, FACE>(r.uy, r.uz, nb.uy, nb.uz) + nb.syz;
   return r;
 }
 
@@ -167,7 +177,7 @@ template <class S> __device__ __forceinline__ void wave1_face(const BcArgs& a, i
     if (cell[c] == 1) copy_raw<S>(a, i, face_slot<T>(a, fid, 1, cell[b]));
     const auto t = load_cell<S>(a, i);
     const auto n = load_cell<S>(a, lin(a, nbr));
-    store_cell<S>(a, i, bc_core(a, face_dr(ax, side), t, n));
+    store_cell<S, true>(a, i, bc_core<S, true>(a, face_dr(ax, side), t, n));
   }
 }
 
@@ -200,9 +210,9 @@ template <class S> __device__ __forceinline__ void wave2_edge(const BcArgs& a, i
       } else {
         n = load_cell<S>(a, lin(a, nbr));
       }
-      t = bc_core(a, face_dr(ak, sk), t, n);
+      t = bc_core<S, false>(a, face_dr(ak, sk), t, n);
     }
-    store_cell<S>(a, i, t);
+    store_cell<S, false>(a, i, t);
   }
 }
 
@@ -227,9 +237,9 @@ template <class S> __device__ __forceinline__ void wave3_corner(const BcArgs& a,
     } else {
       n = load_cell<S>(a, lin(a, nbr));
     }
-    t = bc_core(a, face_dr(ax, sd[ax]), t, n);
+    t = bc_core<S, false>(a, face_dr(ax, sd[ax]), t, n);
   }
-  store_cell<S>(a, i, t);
+  store_cell<S, false>(a, i, t);
 }
 
 // ---------------------------------------------------------------- one pass
@@ -243,9 +253,9 @@ template <class S> struct Cell {
     for (int k = 0; k < 10; ++k) p[k * a.N + i] = v[k];
   }
   __device__ __forceinline__ Mom3<typename S::R> moments(const BcArgs& a) const { return load_slot<S>(a, v); }
-  __device__ __forceinline__ void set(const BcArgs& a, long long i, const Mom3<typename S::R>& m) {  // as store_cell
+  template <bool FACE> __device__ __forceinline__ void set(const BcArgs& a, long long i, const Mom3<typename S::R>& m) {  // as store_cell
     typename S::R raw[10];
-    encode_cell<S>(m, a.sc, raw);
+    encode_cell<S, FACE>(m, a.sc, raw);
 #pragma unroll
     for (int k = 0; k < 10; ++k) v[k] = S::from_r(raw[k], unsigned(k * a.N + i));
   }
@@ -259,7 +269,7 @@ template <class S> __device__ __forceinline__ Mom3<typename S::R> face_value(con
   const int dr = face_dr(ax, side);
   const auto n = load_cell<S>(a, lin(a, nbr));
   const auto t = a.bc_type[dr] == 0 || a.bc_type[dr] == 1 ? n : load_cell<S>(a, lin(a, cell));
-  return bc_core(a, dr, t, n);
+  return bc_core<S, true>(a, dr, t, n);
 }
 
 template <class S> __device__ __forceinline__ void pass_face(const BcArgs& a, int fid, long long first, long long stride) {
@@ -273,7 +283,7 @@ template <class S> __device__ __forceinline__ void pass_face(const BcArgs& a, in
     cell[ax] = side ? a.n[ax] - 1 : 0;
     cell[b] = 2 + int(k / nc);
     cell[c] = 2 + int(k % nc);
-    store_cell<S>(a, lin(a, cell), face_value<S>(a, ax, side, cell));
+    store_cell<S, true>(a, lin(a, cell), face_value<S>(a, ax, side, cell));
   }
 }
 
@@ -295,12 +305,12 @@ template <class S> __device__ __forceinline__ void pass_edge(const BcArgs& a, in
     at[f] = lin(a, rim);
     Cell<S> old;
     old.load(a, at[f]);
-    fresh[f].set(a, at[f], face_value<S>(a, af[1 - f], sd[1 - f], rim));
-    t = bc_core(a, face_dr(af[f], sd[f]), t, (sd[f] == 0 ? old : fresh[f]).moments(a));
+    fresh[f].template set<true>(a, at[f], face_value<S>(a, af[1 - f], sd[1 - f], rim));
+    t = bc_core<S, false>(a, face_dr(af[f], sd[f]), t, (sd[f] == 0 ? old : fresh[f]).moments(a));
   }
   fresh[0].store(a, at[0]);
   fresh[1].store(a, at[1]);
-  store_cell<S>(a, lin(a, cell), t);
+  store_cell<S, false>(a, lin(a, cell), t);
 }
 
 // Corner `corner` (bits x, y, z sides) by one warp: lane q < 3 the face cell next to it on face q and
@@ -325,16 +335,16 @@ template <class S> __device__ __forceinline__ void pass_corner(const BcArgs& a, 
     edge_at = lin(a, ec);
     buf.face_old[lane].load(a, face_at);
     buf.edge_old[lane].load(a, edge_at);
-    buf.face_new[lane].set(a, face_at, face_value<S>(a, lane, sd[lane], fc));
+    buf.face_new[lane].template set<true>(a, face_at, face_value<S>(a, lane, sd[lane], fc));
   }
   __syncwarp();
   if (lane < 3) {
     const int o1 = lane == 0 ? 1 : 0, o2 = lane == 2 ? 1 : 2;
     // the neighbour through face o1 lies on face o2 and the other way round
     auto t = buf.edge_old[lane].moments(a);
-    t = bc_core(a, face_dr(o1, sd[o1]), t, (sd[o1] == 0 ? buf.face_old[o2] : buf.face_new[o2]).moments(a));
-    t = bc_core(a, face_dr(o2, sd[o2]), t, (sd[o2] == 0 ? buf.face_old[o1] : buf.face_new[o1]).moments(a));
-    buf.edge_new[lane].set(a, edge_at, t);
+    t = bc_core<S, false>(a, face_dr(o1, sd[o1]), t, (sd[o1] == 0 ? buf.face_old[o2] : buf.face_new[o2]).moments(a));
+    t = bc_core<S, false>(a, face_dr(o2, sd[o2]), t, (sd[o2] == 0 ? buf.face_old[o1] : buf.face_new[o1]).moments(a));
+    buf.edge_new[lane].template set<false>(a, edge_at, t);
   }
   __syncwarp();
   if (lane == 0) {
@@ -342,8 +352,8 @@ template <class S> __device__ __forceinline__ void pass_corner(const BcArgs& a, 
     auto t = load_cell<S>(a, i);
 #pragma unroll
     for (int ax = 0; ax < 3; ++ax)
-      t = bc_core(a, face_dr(ax, sd[ax]), t, (sd[ax] == 0 ? buf.edge_old[ax] : buf.edge_new[ax]).moments(a));
-    store_cell<S>(a, i, t);
+      t = bc_core<S, false>(a, face_dr(ax, sd[ax]), t, (sd[ax] == 0 ? buf.edge_old[ax] : buf.edge_new[ax]).moments(a));
+    store_cell<S, false>(a, i, t);
   }
   if (lane < 3) {
     buf.face_new[lane].store(a, face_at);

@@ -1,14 +1,13 @@
-// D3Q27 stream-collide in bfloat16 storage, and in float16 with diagnostics or walls (sm_100a):
-// populations exchanged through a shared-memory mailbox, paired-plane arithmetic.
+// D3Q27 stream-collide in the 16-bit storages (sm_100a): populations exchanged through a shared-memory
+// mailbox, paired-plane arithmetic.
 //
-// The other storages run the sweeps of d3q27_sweep.cuh, which are faster (256^3 float16: 0.262
-// against 0.353 ms). A 16-bit store rounds with random bits hashed from the value, so any change of
-// summation order draws new noise. bfloat16 keeps 8 bits: after two steps the stored fields of the two
-// kernels differ by 1.7 % of their norm, more than a caller comparing fields between versions can
-// pass; and a binary64 mass summed over a float16 field follows that field's noise in its eighth
-// digit. This kernel keeps those results what they have always been, bit for bit. Walled float16
-// domains are the served ones, which run whole x columns side by side: a lone column takes 1.49 us
-// a plane here and 1.61 us in the sweep kernel (192^3), and nine of them ran 4 % slower there.
+// binary32 and binary64 run the sweeps of d3q27_sweep.cuh. They are faster in float16 too (256^3: 0.262
+// against 0.353 ms), but sum in another order, and a 16-bit store rounds with random bits hashed from
+// the value: any other order draws other noise. After two steps in bfloat16, which keeps 8 bits, the
+// stored fields of the two kernels differ by 1.7 % of their norm, and the binary64 mass of a float16
+// field follows that field's noise in its eighth digit. So one kernel steps a 16-bit field whatever
+// the options of a call are: diagnostics that are sampled now and then, or walls, only observe or bound
+// the flow, and the stored fields and masses are the same from version to version, bit for bit.
 //
 // Staging: one elected thread issues nine tensor-memory-access (TMA) box copies per plane,
 //
@@ -697,13 +696,11 @@ int launch_one(const hl_world3d* w, double vis, const hl_diag* diag, const Maps&
   return HL_OK;
 }
 
-// ALL: periodic steps without diagnostics too
-template <class S, int NS, bool ALL> int dispatch(const hl_world3d* w, double vis, const hl_diag* d, const Maps& maps, cudaStream_t st) {
+template <class S, int NS> int dispatch(const hl_world3d* w, double vis, const hl_diag* d, const Maps& maps, cudaStream_t st) {
   const bool P = w->periodic != 0, F = w->force != nullptr, G = w->flag != nullptr && !P,
              D = d != nullptr && d->scratch != nullptr;
-#define HL_T_CASE(p, f, g, dg)                  \
-  if constexpr (ALL || dg || !p)                \
-    if (P == p && F == f && G == g && D == dg) return launch_one<S, NS, p, f, g, dg>(w, vis, d, maps, st);
+#define HL_T_CASE(p, f, g, dg) \
+  if (P == p && F == f && G == g && D == dg) return launch_one<S, NS, p, f, g, dg>(w, vis, d, maps, st);
   HL_T_CASE(true, false, false, false)
   HL_T_CASE(true, false, false, true)
   HL_T_CASE(true, true, false, false)
@@ -724,8 +721,8 @@ template <class S, int NS, bool ALL> int dispatch(const hl_world3d* w, double vi
 }  // namespace mb
 
 int launch_mailbox(const hl_world3d* w, double vis, const hl_diag* diag, const sw::Maps& maps, cudaStream_t st) {
-  if (w->storage.dtype == HL_F16) return mb::dispatch<StoreF16, 4, false>(w, vis, diag, maps, st);
-  return mb::dispatch<StoreBF16, 4, true>(w, vis, diag, maps, st);
+  if (w->storage.dtype == HL_F16) return mb::dispatch<StoreF16, 4>(w, vis, diag, maps, st);
+  return mb::dispatch<StoreBF16, 4>(w, vis, diag, maps, st);
 }
 
 template <class S>

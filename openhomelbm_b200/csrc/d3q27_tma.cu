@@ -144,16 +144,15 @@ bool box_eligible(const hl_world3d* w) {
 }
 
 int launch_step_tma(const hl_world3d* w, double vis, const hl_diag* diag, cudaStream_t st) {
-  // bfloat16, float16 with diagnostics and walled float16: see d3q27_mailbox.cu
+  // the 16-bit storages, whatever the call's options: see d3q27_mailbox.cu
   const hl_dtype dt = w->storage.dtype;
-  const bool mailbox = dt == HL_BF16 || (dt == HL_F16 && (!w->periodic || (diag != nullptr && diag->scratch != nullptr)));
+  const bool mailbox = dt == HL_F16 || dt == HL_BF16;
   sw::Maps maps;
   const int rc = tma::encode_maps(w, mailbox, &maps);
   if (rc != HL_OK) return rc;
   if (mailbox) return launch_mailbox(w, vis, diag, maps, st);
   switch (dt) {
     case HL_F32: return sw::dispatch<StoreF32, true>(w, vis, diag, maps, st);
-    case HL_F16: return sw::dispatch<StoreF16, true>(w, vis, diag, maps, st);
     case HL_F64: return sw::dispatch<StoreF64, true>(w, vis, diag, maps, st);
     default: break;
   }

@@ -70,3 +70,53 @@ BOUNDARY = {
 @pytest.mark.parametrize("shape,storage,types", list(BOUNDARY))
 def test_boundary_cells(shape, storage, types):
     assert boundary(shape, storage, types) == BOUNDARY[shape, storage, types]
+
+
+def step(shape, storage, periodic, force, diagnostics):
+    """Three steps of a box or a duct: the digest of the field."""
+    from openhomelbm_b200.lbm3d import LBM_Solver3D
+
+    s = LBM_Solver3D(*shape, periodic=periodic, storage=storage, with_force=force, use_graph=False, u_scale=U_SCALE,
+                     s_scale=S_SCALE)
+    f = s.flows[0]
+    s.set_viscosity(0.01)
+    for m in f.moments:
+        m.copy_(_field(shape, storage, 5))
+    if force:
+        f.force.copy_(torch.tensor(np.random.default_rng(6).uniform(-1e-4, 1e-4, (3, *shape)).astype(np.float32)))
+        f.use_force = True
+    if not periodic:
+        f.bc_type = [0, 1, 1, 1, 1, 1]
+        f.bc_value = np.array([(0.04, 0, 0)] + [(0, 0, 0)] * 5, np.float32)
+    s.diagnostics = diagnostics
+    for _ in range(3):
+        s.step()
+    torch.cuda.synchronize()
+    return _digest(f.cur)
+
+
+STEP = {
+    ((20, 32, 64), "float16", True, False): "d8987bf971396272",
+    ((20, 32, 64), "float16", True, True): "7f44aced4c7b225a",
+    ((20, 32, 64), "float16", False, False): "71d00ccf95703bd5",
+    ((20, 32, 64), "float16", False, True): "705caeb7ab2054ec",
+    ((20, 32, 64), "bfloat16", True, False): "cf09f35fab4bfc42",
+    ((20, 32, 64), "bfloat16", True, True): "b12f34e3b93cd8ca",
+    ((20, 32, 64), "bfloat16", False, False): "6c391ffd3af4bdb3",
+    ((20, 32, 64), "bfloat16", False, True): "fd6d183feaf6fe49",
+    ((33, 16, 32), "float16", True, False): "f058b6715e26a9c9",
+    ((33, 16, 32), "float16", True, True): "aa305854f378882e",
+    ((33, 16, 32), "float16", False, False): "18dab52d69596c77",
+    ((33, 16, 32), "float16", False, True): "84b8ae5c3055d015",
+    ((33, 16, 32), "bfloat16", True, False): "29435933b7f3f62b",
+    ((33, 16, 32), "bfloat16", True, True): "443566c383fb3d2b",
+    ((33, 16, 32), "bfloat16", False, False): "739bc518d1054f09",
+    ((33, 16, 32), "bfloat16", False, True): "b16da01627ffcfcd",
+}
+
+
+@pytest.mark.parametrize("diagnostics", [False, True])
+@pytest.mark.parametrize("shape,storage,periodic,force", list(STEP))
+def test_steps_with_and_without_diagnostics(shape, storage, periodic, force, diagnostics):
+    """The mass and health sums observe: the stored field is the same with them and without."""
+    assert step(shape, storage, periodic, force, diagnostics) == STEP[shape, storage, periodic, force]

@@ -577,16 +577,23 @@ __device__ __forceinline__ float4 segment_of(const World& w, int j) {
   return make_float4(tf[2 * n], tf[2 * n + 1], tf[2 * n1], tf[2 * n1 + 1]);
 }
 
-// get_cutcell over a candidate list, segments cand[k] in any order, holding every segment of a near
-// solid that can cross a link of the cell. The per-segment arithmetic is get_cutcell's, and of
-// equally near crossings the lowest segment wins as in its ascending loop, so the result is the same.
-// segs: the world's segments in shared memory, or NULL.
+constexpr int BAND_CAND = 16;         // candidate segments kept per cell; more: the full scan
+
+// get_cutcell over a candidate list, segments cand[k] in any order (many threads note them, and the order
+// changes from run to run), holding every segment of a near solid that can cross a link of the cell.
+// The per-segment arithmetic is get_cutcell's, and of equally near crossings the lowest segment wins as
+// in its ascending loop. What that loop finds depends on the order in one case more: a crossing at the
+// cell's own point whose t rounds below zero, or is NaN, is kept or replaced by what comes after it. With
+// such a crossing, as with more candidates than the list holds, get_cutcell itself decides. segs: the
+// world's segments in shared memory, or NULL. (Sorting each list first took 0.7 of 24.6 us for the
+// 512 x 128 wake and 20 of 1970 for 60 worlds.)
 __device__ __forceinline__ Cut get_cutcell_list(const World& w, const float4* segs, const int* cand, int nc, float x,
                                                 float y, float dx, float dy) {
   Cut r{-1.f, -1.f, -1, -1};
   int best = 0x7fffffff;
+  bool scan = nc > BAND_CAND;
   const float ax = x - dx, ay = y - dy, bx = x, by = y;
-  for (int k = 0; k < nc; ++k) {
+  for (int k = 0; k < nc && !scan; ++k) {
     const int j = cand[k];
     const float4 g = segs ? segs[j] : segment_of(w, j);
     const float cx = g.x, cy = g.y, ex = g.z, ey = g.w;
@@ -597,12 +604,14 @@ __device__ __forceinline__ Cut get_cutcell_list(const World& w, const float4* se
     const float cdb = cda + abc - abd;
     if (cda * cdb > 0.f) continue;
     const float t = 1.f - cda / (abd - abc);
+    scan = !(t >= 0.f);
     if (r.t < 0.f || t < r.t || (t == r.t && j < best)) {
       best = j;
       r.t = t;
       r.ratio = abc / (abc - abd);
     }
   }
+  if (scan) return get_cutcell(w, x, y, dx, dy);
   if (r.t >= 0.f) {
     r.solid = best / w.max_segments;
     r.seg = best - r.solid * w.max_segments;
@@ -612,7 +621,6 @@ __device__ __forceinline__ Cut get_cutcell_list(const World& w, const float4* se
 
 constexpr int BAND_SEGS = 1024;       // segments staged per block
 constexpr int BAND_CELLS = 128;       // cells of a block's pass
-constexpr int BAND_CAND = 16;         // candidate segments kept per cell; more: the full scan
 constexpr int BAND_BLOCKS = 96;       // blocks per world, fewer where many worlds share the chip
 
 // The cells near a solid. Only a few cells of a block lie next to an outline, and a cut cell is nine
@@ -728,9 +736,7 @@ template <class S, int THREADS> __global__ void __launch_bounds__(THREADS) band_
           const Mom2<R> mn = load2<S>(w, N, (long long)xn * w.ny + yn, cur);
           const Mom2<R> me = load2<S>(w, N, (long long)cx * w.ny + cy, cur);
           const int nc = s_count[at];
-          const Cut cc = nc > BAND_CAND ? get_cutcell(w, float(cx), float(cy), float(dx), float(dy))
-                                        : get_cutcell_list(w, segs, s_cand + at * BAND_CAND, nc, float(cx), float(cy),
-                                                           float(dx), float(dy));
+          const Cut cc = get_cutcell_list(w, segs, s_cand + at * BAND_CAND, nc, float(cx), float(cy), float(dx), float(dy));
           if (cc.t >= 0.f && cc.solid >= 0) {
             s_cut[at] = 1;
             const int s = cc.solid, nseg = s_nseg[s];

@@ -1,7 +1,10 @@
-"""The outline reads of the D2Q9 cut-link kernel (csrc/d2q9.cu), compiled from that file for the CPU.
+"""Functions of the D2Q9 cut-link kernel (csrc/d2q9.cu), compiled from that file for the CPU.
 
 band_kernel stages segment_of(w, j) for every slot of every solid, used or not. The reads must stay
 inside the world's vertex array [n_objects][max_segments][2]: here it ends at an unreadable page.
+
+A cell's candidate segments are noted in any order. The cut found from them must be the one that
+get_cutcell finds over all segments in their order.
 """
 import os
 import re
@@ -74,6 +77,72 @@ int main(int argc, char** argv) {
 def test_staging_reads_only_the_outline_array(tmp_path, max_segments, counts):
     r = run(tmp_path, function("segment_of") + MAIN, max_segments, *counts)
     assert r.returncode == 0, (r.returncode, r.stderr)
+
+
+SEARCH = """
+#include <algorithm>
+#include <random>
+#include <vector>
+constexpr int BAND_CAND = 16;
+struct Cut {
+  float t, ratio;
+  int solid, seg;
+};
+"""
+
+# Two or three solids of one segment each (an outline of two vertices, there and back): the first crosses a
+# link at the cell's own point with t < 0, the others cross it further on. Every order of the
+# candidates, and both orders of the solids.
+SEARCH_MAIN = """
+int main() {
+  std::mt19937 g(1);
+  auto uni = [&](float a, float b) { return std::uniform_real_distribution<float>(a, b)(g); };
+  int found = 0, wrong = 0;
+  for (long trial = 0; trial < 3000000 && found < 300; ++trial) {
+    const float x = float(g() % 500 + 2), y = float(g() % 500 + 2);
+    const int d = g() % 8, dx = (d < 4 ? d : d + 1) / 3 - 1, dy = (d < 4 ? d : d + 1) % 3 - 1;
+    const float a = uni(0.f, 6.2831853f), l0 = uni(.05f, 2.f), l1 = uni(.05f, 2.f);
+    const float s0[4] = {x + l0 * cosf(a), y + l0 * sinf(a), x - l1 * cosf(a), y - l1 * sinf(a)};
+    const int n = 2 + int(g() % 2);
+    for (int turned = 0; turned < 2; ++turned) {
+      float tf[3 * 4], position[6] = {x, y, x, y, x, y}, scale[3] = {1, 1, 1}, radius[3] = {100, 100, 100};
+      const int line_num[3] = {2, 2, 2};
+      for (int s = 0; s < n; ++s) {
+        const float by = s == 0 ? 0.f : s == 1 ? .3f : .6f;
+        float* t = tf + 4 * (turned ? n - 1 - s : s);
+        for (int k = 0; k < 4; ++k) t[k] = s0[k] - by * float(k & 1 ? dy : dx);
+      }
+      World w{n, 2, 1, line_num, tf, position, scale, radius};
+      World alone = w;
+      alone.n_objects = 1;
+      alone.tf = turned ? tf + 4 * (n - 1) : tf;
+      const Cut near = get_cutcell(alone, x, y, float(dx), float(dy));
+      if (!(near.solid >= 0 && near.t < 0.f)) continue;
+      ++found;
+      const Cut want = get_cutcell(w, x, y, float(dx), float(dy));
+      std::vector<int> order(2 * n);
+      for (int k = 0; k < 2 * n; ++k) order[k] = k;
+      do {
+        int cand[6];
+        std::copy(order.begin(), order.end(), cand);
+        const Cut got = get_cutcell_list(w, nullptr, cand, 2 * n, x, y, float(dx), float(dy));
+        wrong += got.t != want.t || (want.t >= 0.f && (got.solid != want.solid || got.seg != want.seg || got.ratio != want.ratio));
+      } while (std::next_permutation(order.begin(), order.end()));
+    }
+  }
+  printf("%d near crossings, %d wrong cuts\\n", found, wrong);
+  return found < 20 ? 3 : wrong ? 2 : 0;
+}
+"""
+
+
+@pytest.mark.parametrize("flags", [(), ("-mfma", "-ffp-contract=fast")])
+def test_cut_does_not_depend_on_the_candidates_order(tmp_path, flags):
+    if flags and "fma" not in open("/proc/cpuinfo").read():
+        pytest.skip("no fused multiply-add on this CPU")
+    body = "#include <cmath>\n" + SEARCH + function("segment_of") + function("get_cutcell") + function("get_cutcell_list")
+    r = run(tmp_path, body + SEARCH_MAIN, flags=flags)
+    assert r.returncode == 0, (r.returncode, r.stdout, r.stderr)
 
 
 @pytest.mark.gpu

@@ -220,8 +220,8 @@ template <> struct Range<double> {
     for (int k = 4; k < 10; ++k) s = max(s, hi(m[k]));
   }
   template <bool ENC> __device__ __forceinline__ bool clamps(const Scale&, bool n = ENC) const {
-    // the next larger high word bounds every value with this one
-    const double U = __hiloint2double(int(u + 1), 0), q = __hiloint2double(int(s + 1), 0);
+    // the largest value with this high word: NaN for the high words of infinity and of every NaN
+    const double U = __hiloint2double(int(u), -1), q = __hiloint2double(int(s), -1);
     return !((n ? 6.0 * U * U + 12.0 * q <= 0.6 : 4.5 * U * U + 12.0 * q <= 0.45) && d < 0x40000000u);  // 0 <= rho < 2
   }
 };

@@ -113,7 +113,8 @@ typedef struct {
 } hl_bc3d;
 
 /* Scratch for the diagnostics of one step: per-CTA partial sums and a completion counter.
- * Size it with hl_d3q27_scratch_bytes(); zero it once before first use. */
+ * Size it with hl_d3q27_scratch_bytes(); zero it once before first use. The least is 64 bytes and
+ * 12 bytes per SM; less is rejected with HL_ERR_ARG. */
 typedef struct {
   void* scratch;
   size_t scratch_bytes;
@@ -151,7 +152,7 @@ HL_API size_t hl_d3q27_scratch_bytes(const hl_world3d* w);
  *    float64 (other storages return HL_ERR_ARG); it always runs the kernels that take rows of
  *    any length, never a TMA-staged one, so its results can differ from hl_d3q27_stream_collide in
  *    rounding.
- *  - Limit: 64 + 12 bytes for each of two CTAs per SM, i.e. devices with up to 680 SMs (a B200 has
+ *  - Limit: 16 bytes and 12 bytes per SM of scratch, i.e. devices with up to 1364 SMs (a B200 has
  *    148); larger needs are rejected with HL_ERR_ARG.
  *  - The first call on a device resolves the array's device address (cudaGetSymbolAddress,
  *    with that device current); make that first call before any stream capture.

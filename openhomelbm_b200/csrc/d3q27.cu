@@ -35,6 +35,7 @@
 // HBM traffic is one read and one write of the 10 moments per cell (80 B in binary32).
 // Halo reloads come from L2 because all CTAs march the same x range in step.
 
+#include <algorithm>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -267,14 +268,19 @@ template <int TY> Plan make_plan(int nx, int ny, int nz) {
   return p;
 }
 
-// one partial sum and one count per block, after the completion counter
+// Diagnostics scratch: the completion counter (16 bytes), then slots of one partial sum and one count. A
+// block has a slot of its own where there are as many; the least is one slot per SM, which the sweeps'
+// two blocks per SM share (two sums in a slot give the same bits in either order).
 size_t diag_scratch_bytes() { return size_t(sw::BLOCKS_PER_SM) * num_sms() * (sizeof(double) + sizeof(int)) + 64; }
+static size_t diag_scratch_least() { return size_t(num_sms()) * (sizeof(double) + sizeof(int)) + 64; }
 
 void fill_diag(StepArgs& a, const hl_diag* diag) {
   char* s = static_cast<char*>(diag->scratch);
+  const size_t room = (diag->scratch_bytes - 16) / (sizeof(double) + sizeof(int));
+  a.diag_slots = int(std::min(room, size_t(sw::BLOCKS_PER_SM) * num_sms()));
   a.counter = reinterpret_cast<unsigned*>(s);
   a.partials = reinterpret_cast<double*>(s + 16);
-  a.bad_partials = reinterpret_cast<int*>(s + 16 + sizeof(double) * sw::BLOCKS_PER_SM * num_sms());
+  a.bad_partials = reinterpret_cast<int*>(s + 16 + sizeof(double) * a.diag_slots);
   a.mass = diag->mass;
   a.health = diag->health;
 }
@@ -349,9 +355,9 @@ extern "C" int hl_d3q27_stream_collide(const hl_world3d* w, double vis_shear, co
   HL_CHECK_ARG(w->nx >= 1 && w->ny >= 1 && w->nz >= 1, "d3q27: bad dims %d x %d x %d", w->nx, w->ny, w->nz);
   HL_CHECK_ARG(w->cur != nullptr && w->post != nullptr && w->cur != w->post, "d3q27: cur/post must be distinct");
   HL_CHECK_ARG(vis_shear > 0.0f, "d3q27: viscosity must be positive");
-  HL_CHECK_ARG(diag == nullptr || diag->scratch == nullptr || diag->scratch_bytes >= d3::diag_scratch_bytes(),
+  HL_CHECK_ARG(diag == nullptr || diag->scratch == nullptr || diag->scratch_bytes >= d3::diag_scratch_least(),
                "d3q27: diagnostics scratch too small (%zu < %zu)", diag ? diag->scratch_bytes : 0,
-               d3::diag_scratch_bytes());
+               d3::diag_scratch_least());
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (g_tune_d3_kernel == 2 && !d3::tma_eligible(w)) {
     set_error("d3q27: the TMA kernel needs ny %% 16 == 0, nz %% 32 == 0 and a non-float64 storage");
@@ -381,7 +387,7 @@ extern "C" size_t hl_d3q27_scratch_bytes(const hl_world3d*) { return d3::diag_sc
 namespace hl {
 namespace d3 {
 
-constexpr size_t kNoAllocScratchBytes = 16384;  // 64 + 12 bytes per CTA, two CTAs per SM: up to 680 SMs
+constexpr size_t kNoAllocScratchBytes = 16384;  // 16 + 12 bytes per CTA, one CTA per SM or more: up to 1364 SMs
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratchBytes];
 
 // Device address of g_noalloc_scratch on the current device. The host-side symbol is only a
@@ -421,7 +427,7 @@ extern "C" int hl_d3q27_stream_collide_noalloc(const hl_world3d* w, double vis_s
   HL_CHECK_ARG(vis_shear > 0.0, "d3q27 (no-alloc): viscosity must be positive");
   HL_CHECK_ARG(w->storage.dtype == HL_F32 || w->storage.dtype == HL_F64,
                "d3q27 (no-alloc): storage must be float32 or float64");
-  const size_t need = d3::diag_scratch_bytes();
+  const size_t need = 16 + size_t(d3::num_sms()) * (sizeof(double) + sizeof(int));
   HL_CHECK_ARG(need <= d3::kNoAllocScratchBytes,
                "d3q27 (no-alloc): needs %zu bytes of scratch for %d SMs; the static scratch holds %zu", need,
                d3::num_sms(), d3::kNoAllocScratchBytes);

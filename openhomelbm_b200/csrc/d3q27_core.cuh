@@ -21,6 +21,7 @@ struct StepArgs {
   Scale sc;
   double* partials;        // [gridDim.x] mass partials
   int* bad_partials;       // [gridDim.x]
+  int diag_slots;  // partial sums and counts that the diagnostics scratch holds
   unsigned* counter;       // completion counter (returns to 0 after each launch)
   double* mass;
   int* health;

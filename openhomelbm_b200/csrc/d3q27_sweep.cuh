@@ -1136,8 +1136,13 @@ __global__ void __launch_bounds__(THREADS, MINB)
     const int bs = block_sum<int>(bad, red_i);
     __shared__ bool last;
     if (tid == 0) {
-      a.partials[blockIdx.x] = ms;
-      a.bad_partials[blockIdx.x] = bs;
+      if (gridDim.x <= unsigned(a.diag_slots)) {
+        a.partials[blockIdx.x] = ms;
+        a.bad_partials[blockIdx.x] = bs;
+      } else {  // two blocks a slot at most
+        atomicAdd(&a.partials[blockIdx.x % unsigned(a.diag_slots)], ms);
+        atomicAdd(&a.bad_partials[blockIdx.x % unsigned(a.diag_slots)], bs);
+      }
       __threadfence();
       last = atomicAdd(a.counter, 1u) == gridDim.x - 1;
     }
@@ -1146,7 +1151,7 @@ __global__ void __launch_bounds__(THREADS, MINB)
       __threadfence();
       double tot = 0.0;
       int tb = 0;
-      for (unsigned b = tid; b < gridDim.x; b += THREADS) {
+      for (unsigned b = tid; b < min(gridDim.x, unsigned(a.diag_slots)); b += THREADS) {
         tot += __ldcg(&a.partials[b]);
         tb += __ldcg(&a.bad_partials[b]);
       }
@@ -1216,8 +1221,12 @@ int launch(const hl_world3d* w, double vis, const hl_diag* diag, const Maps& map
   auto kern = sweep_kernel<S, TMA, NST, BLOCKS_PER_SM, PERIODIC, FORCE, FLAGS, DIAG, false>;
   const int rc = set_smem_attr(reinterpret_cast<const void*>(kern), SMEM, "cudaFuncSetAttribute(d3q27 stream_collide)");
   if (rc != HL_OK) return rc;
-  const int slots = BLOCKS_PER_SM * num_sms();
-  kern<<<a.n_items < slots ? a.n_items : slots, THREADS, SMEM, st>>>(a, maps, nullptr, 0, 0);
+  const int slots = BLOCKS_PER_SM * num_sms(), grid = a.n_items < slots ? a.n_items : slots;
+  if (DIAG && grid > a.diag_slots) {  // blocks add to shared slots
+    const cudaError_t e = cudaMemsetAsync(a.partials, 0, size_t(a.diag_slots) * (sizeof(double) + sizeof(int)), st);
+    if (e != cudaSuccess) return cuda_status(e, "d3q27 stream_collide: clear partial sums");
+  }
+  kern<<<grid, THREADS, SMEM, st>>>(a, maps, nullptr, 0, 0);
   HL_LAUNCH_CHECK("d3q27 stream_collide launch");
   return HL_OK;
 }

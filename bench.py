@@ -751,7 +751,7 @@ def main():
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--kernel", type=int, default=0, help="0 auto, 1 async-copy kernel, 2 TMA kernel")
     ap.add_argument("--chunks", type=int, default=0, help="x split per tile column (0 automatic)")
-    ap.add_argument("--stages", type=int, default=0, help="TMA pipeline stages (0 automatic)")
+    ap.add_argument("--stages", type=int, default=0, help="planes staged by the kernel of the 16-bit storages (0 automatic)")
     ap.add_argument("--workload", default="tgv", choices=["tgv", "precision", "serve", "karman", "batch"],
                     help="tgv: the headline throughput line; precision: float64/32/16/bf16 accuracy form; "
                          "serve: served vs plain mesh-coupled domains; karman: D2Q9 wake vs the oracle; "

@@ -14,6 +14,7 @@ namespace hl {
 static thread_local char g_err[512] = "";
 int g_tune_d3_kernel = 0;
 int g_tune_d3_chunks = 0;
+int g_tune_d3_stages = 0;
 int g_tune_d3_link_blocks = 0;
 
 void set_error(const char* fmt, ...) {
@@ -78,7 +79,8 @@ extern "C" int hl_set_tuning(const char* key, int value) {
     return HL_OK;
   }
   if (!strcmp(key, "d3q27_stages") && (value == 0 || (value >= 3 && value <= 5))) {
-    return HL_OK;  // the staging depth is fixed per storage type
+    hl::g_tune_d3_stages = value;
+    return HL_OK;
   }
   hl::set_error("hl_set_tuning: unknown key or value (%s = %d)", key, value);
   return HL_ERR_ARG;

@@ -720,9 +720,19 @@ template <class S, int NS> int dispatch(const hl_world3d* w, double vis, const h
 
 }  // namespace mb
 
+template <int NS>
+static int launch_depth(const hl_world3d* w, double vis, const hl_diag* diag, const sw::Maps& maps, cudaStream_t st) {
+  if (w->storage.dtype == HL_F16) return mb::dispatch<StoreF16, NS>(w, vis, diag, maps, st);
+  return mb::dispatch<StoreBF16, NS>(w, vis, diag, maps, st);
+}
+
+// 4 staged planes (the pair being computed and the next pair) unless tuned
 int launch_mailbox(const hl_world3d* w, double vis, const hl_diag* diag, const sw::Maps& maps, cudaStream_t st) {
-  if (w->storage.dtype == HL_F16) return mb::dispatch<StoreF16, 4>(w, vis, diag, maps, st);
-  return mb::dispatch<StoreBF16, 4>(w, vis, diag, maps, st);
+  switch (g_tune_d3_stages) {
+    case 3: return launch_depth<3>(w, vis, diag, maps, st);
+    case 5: return launch_depth<5>(w, vis, diag, maps, st);
+    default: return launch_depth<4>(w, vis, diag, maps, st);
+  }
 }
 
 template <class S>

@@ -15,6 +15,7 @@ void set_error(const char* fmt, ...);
 int cuda_status(cudaError_t e, const char* what);
 extern int g_tune_d3_kernel;  // hl_set_tuning("d3q27_kernel")
 extern int g_tune_d3_chunks;  // hl_set_tuning("d3q27_chunks")
+extern int g_tune_d3_stages;  // hl_set_tuning("d3q27_stages")
 extern int g_tune_d3_link_blocks;  // hl_set_tuning("d3q27_link_blocks")
 
 // Per-device host state (a process may drive several GPUs): the current device's SM count,

@@ -172,6 +172,9 @@ __device__ __forceinline__ P2 reciprocal(P2 x) {
   return r0 * (P2(1.0) - x * r0) + r0;
 }
 __device__ __forceinline__ double reciprocal(double x) { return 1.0 / x; }
+// a * b, never fused into what uses it
+__device__ __forceinline__ P2 mul_rn(P2 a, float b) { return P2(__fmul_rn(a.x(), b), __fmul_rn(a.y(), b)); }
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ P2 bcast(P2, float v) { return P2(v, v); }
 __device__ __forceinline__ double bcast(double, double v) { return v; }
 __device__ __forceinline__ float bcast(float, float v) { return v; }
@@ -592,7 +595,9 @@ template <class S, bool FORCE, class V>
 __device__ __forceinline__ void collide_raw(const Totals<V>& t, const V F[3], const Collide<V>& k, const Scale& sc,
                                               V raw[10], V& rho_out) {
   using R = typename S::R;
-  const V drho = t.z[0] * V(1.0 / 216.0);
+  // -216 exactly where no population arrives: drho -1 and rho 0, which the health count and a step of
+  // such a cell need, if the product is rounded before the sum (fused, rho is the constant's error)
+  const V drho = mul_rn(t.z[0], R(1.0 / 216.0));
   const V rho = drho + V(1.0);
   const V inv = reciprocal(rho);
   const V i216 = inv * V(1.0 / 216.0);

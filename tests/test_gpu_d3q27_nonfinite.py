@@ -38,3 +38,33 @@ def test_binary64_cells_with_nan_send_nothing(bits, shape, regime):
     got = f.moments[1].cpu().numpy()
     assert np.isfinite(got).all()
     assert np.abs(got - want).max() <= 320 * 2.0 ** -53
+
+
+@pytest.mark.parametrize("storage", ["float32", "float64"])
+@pytest.mark.parametrize("shape", [(8, 16, 64), (8, 17, 36), (8, 11, 33)])
+@pytest.mark.parametrize("periodic", [True, False])
+@pytest.mark.parametrize("state", ["nan", "empty"])
+def test_cells_that_nothing_reaches_are_counted(storage, shape, periodic, state):
+    """A flow that has blown up (NaN everywhere) or a cavity without fluid sends no population: the
+    density of the cells inside is zero, and each counts as unhealthy."""
+    from openhomelbm_b200.lbm3d import LBM_Solver3D
+
+    s = LBM_Solver3D(*shape, periodic=periodic, storage=storage, use_graph=False)
+    f = s.flows[0]
+    s.set_viscosity(0.01)
+    t = torch.tensor(_state(shape, "calm", 4))
+    inside = (slice(2, 6), slice(3, 9), slice(4, 30))  # its inner 2 x 4 x 24 cells hear from no other
+    if state == "nan":
+        t[1:] = float("nan")
+    else:
+        t[(slice(None),) + inside] = 0.0
+    for m in f.moments:
+        m.copy_(t)
+    s.diagnostics = True
+    s.step()
+    nx, ny, nz = shape
+    cells = nx * ny * nz if periodic else (nx - 2) * (ny - 2) * (nz - 2)
+    want = cells if state == "nan" else 2 * 4 * 24
+    assert int(s.health[0]) == want
+    rho = f.cur[0, 3:5, 4:8, 5:29]
+    assert (rho == 0).all(), rho.flatten()[:4]

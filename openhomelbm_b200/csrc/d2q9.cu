@@ -884,8 +884,8 @@ template <class S> __global__ void __launch_bounds__(BC_THREADS) boundary_kernel
       if (tid < 8) {
         const int side = tid >> 1, base = side < 2 ? side * ey : 2 * ey + (side - 2) * ex;
         const int last = (side < 2 ? ey : ex) - 1;
-        if (!(tid & 1)) update(base, &old[tid]);
-        else if (last > 0) update(base + last, &old[tid]);
+        // the lanes of a side's two ends side by side (in two branches the one would wait for the other)
+        if (!(tid & 1) || last > 0) update(base + (tid & 1 ? last : 0), &old[tid]);
       }
       __syncwarp();
       if (tid < 4) {

@@ -433,6 +433,7 @@ typedef struct {
 #define HL_PHASE_STREAM 2   /* stream_and_collide (lbm_func.py:322-467) incl. cut links and loads */
 #define HL_PHASE_BC 4       /* apply_bc (lbm_func.py:610-682) + binary32 load copies */
 #define HL_PHASE_ALL 7
+#define HL_PHASE_SAME_SIZE 8 /* hl_d2q9_step_batch, added to phases: every world is max_nx x max_ny */
 
 /* Replaces one LBM_Solver.step (envs/lbm/lbm_solver.py:97-141) of one world: segments,
  * stream_and_collide with polygon cut cells and momentum exchange, apply_bc. solids may be

@@ -16,6 +16,7 @@ LIB_PATH = os.path.join(HERE, "libhomelbm.so")
 HL_OK, HL_ERR_ARG, HL_ERR_UNSUPPORTED, HL_ERR_CUDA, HL_ERR_TIMEOUT = 0, -1, -2, -3, -4
 HL_F32, HL_F16, HL_BF16, HL_F64 = 0, 1, 2, 3
 HL_PHASE_SEGMENTS, HL_PHASE_STREAM, HL_PHASE_BC, HL_PHASE_ALL = 1, 2, 4, 7
+HL_PHASE_SAME_SIZE = 8
 
 
 class HomeLBMError(RuntimeError):

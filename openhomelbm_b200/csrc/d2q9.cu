@@ -1086,9 +1086,19 @@ template <class S, int TX> int grid_strips(const d2::Launch& L, long long total,
 //   64 of 256 x 200                90.6 /  86.1  73.7  64.6  52.8    binary16  105.8 / 75.3 65.3 55.1 58.6
 //   4096 x 2048                     206 /   204   169   152   112
 //   2048 x 2048 binary64            151 /   132   116   109   105
-template <class S> int stream_grid(const d2::Launch& L, int n, int maxx, int maxy, cudaStream_t st) {
+// Of worlds of different sizes only the largest sides are known here, and most strips cut from them may lie
+// past the worlds: the few that do not would be long ones with the chip half empty. Without the caller's
+// word that all sizes are the same, eight times as many are asked for. us, a thread per cell / as
+// many as for worlds of one size / twice / 4 / 8 / 16 times:
+//   one 512 x 512 and 23 of 32 x 32          20.7 /  26.4  26.8  17.4  16.1  18.9
+//   8 of 64 .. 512 x 48 .. 400               11.2 /  15.7   9.3  11.2  11.2  11.3
+//   24 of the same                           22.6 /  36.4  22.4  19.1  21.3  22.9
+//   two of 2048 x 16 and two of 16 x 1024    18.2 /  28.6  28.2  28.4  18.3  15.2
+//   one 1500 x 400 and 7 of 300 x 80         27.3 /  29.3  29.0  22.5  21.6  23.3
+//   60 of 256 .. 1024 x 128 .. 512          270.7 / 154.7 152.5 152.5 152.3 169.9
+template <class S> int stream_grid(const d2::Launch& L, int n, int maxx, int maxy, bool even, cudaStream_t st) {
   const int sy = (maxy + d2::STRIP_Y - 1) / d2::STRIP_Y;
-  const long long least = 15ll * device_sms();
+  const long long least = (even ? 15ll : 8 * 15ll) * device_sms();
   auto strips = [&](int tx) { return (long long)n * sy * ((maxx + tx - 1) / tx); };
   if (strips(4) < least || strips(4) > 0x7fffffffll) {
     dim3 grid((maxy + 31) / 32, (maxx + 7) / 8, n);
@@ -1113,7 +1123,7 @@ template <class S> int run_phases(const d2::Launch& L, int n, int maxx, int maxy
       const int rc = stream_tiles<S>(L, *tw, st);
       if (rc != HL_OK) return rc;
     } else {
-      const int rc = stream_grid<S>(L, n, maxx, maxy, st);
+      const int rc = stream_grid<S>(L, n, maxx, maxy, n == 1 || (phases & HL_PHASE_SAME_SIZE) != 0, st);
       if (rc != HL_OK) return rc;
     }
     if (any_solid) {

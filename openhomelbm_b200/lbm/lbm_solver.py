@@ -122,8 +122,8 @@ class LBM_Solver:
     def _launch(self, parity: int, stream) -> None:
         f0 = self.flows[0]
         _lib.check(_lib.lib().hl_d2q9_step_batch(_lib.ptr(self._desc_dev), self.nworld, parity, f0.storage_code,
-                                                 self.nx, self.ny, int(self._any_solid), _lib.HL_PHASE_ALL,
-                                                 stream), "LBM_Solver.step")
+                                                 self.nx, self.ny, int(self._any_solid),
+                                                 _lib.HL_PHASE_ALL | _lib.HL_PHASE_SAME_SIZE, stream), "LBM_Solver.step")
 
     def step(self) -> None:
         """Advance every world by one step (reference: LBM_Solver.step, lbm_solver.py:97-141)."""

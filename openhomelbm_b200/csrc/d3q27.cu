@@ -1,6 +1,6 @@
-// D3Q27 stream-collide in binary32 for rows of any length, and the entry points of the step. Domains
-// whose rows are multiples of 16 bytes, binary64 and the 16-bit storages run the sweeps of
-// d3q27_sweep.cuh (d3q27_tma.cu; binary64 with other rows from here). For binary32 rows that
+// D3Q27 stream-collide in binary32 for rows of any length, and the entry points of the step. binary32
+// domains whose rows are multiples of 16 bytes and all of binary64 run the sweeps of d3q27_sweep.cuh
+// (d3q27_tma.cu), the 16-bit storages d3q27_mailbox.cu. For binary32 rows that
 // tensor copies cannot take, the sweeps staged by 4-byte asynchronous copies are the slower form
 // (200 x 150 x 133: 188 us a step against 164 us here; 60 x 47 x 53: 15.4 against 11.3): a warp of 16
 // column pairs stores such rows in parts of sectors, and this kernel's warps store whole rows.
@@ -45,30 +45,27 @@
 namespace hl {
 namespace d3 {
 
-constexpr int TZ = 32;
-constexpr int BZ = TZ + 2;
+constexpr int TY = 16, TZ = 32;
+constexpr int BY = TY + 2, BZ = TZ + 2;
 constexpr int NSTAGE = 3;
+constexpr int NSRC = BY * BZ;
+constexpr int NDST = TY * TZ;
+constexpr int STEP_THREADS = ((NSRC + 31) / 32) * 32;
+constexpr int STEP_SMEM = (NSTAGE * 10 + 27) * NSRC * int(sizeof(float));
 
-template <int TY> struct Tile {
-  static constexpr int BY = TY + 2;
-  static constexpr int NSRC = BY * BZ;
-  static constexpr int NDST = TY * TZ;
-  static constexpr int THREADS = ((NSRC + 31) / 32) * 32;
-};
-
-template <int TY, class S, bool PERIODIC, bool FORCE, bool FLAGS, bool DIAG>
-__global__ void __launch_bounds__(Tile<TY>::THREADS, 1) step_kernel(const StepArgs a) {
-  using T = typename S::T;
-  using R = typename S::R;
-  using TL = Tile<TY>;
+template <bool PERIODIC, bool FORCE, bool FLAGS, bool DIAG>
+__global__ void __launch_bounds__(STEP_THREADS, 1) step_kernel(const StepArgs a) {
+  using S = StoreF32;
+  using T = float;
+  using R = float;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* stage = reinterpret_cast<T*>(smem_raw);  // [NSTAGE][10][NSRC]
-  R* mb = reinterpret_cast<R*>(smem_raw + ((NSTAGE * 10 * TL::NSRC * sizeof(T) + 15) / 16) * 16);  // [27][NSRC]
+  R* mb = stage + NSTAGE * 10 * NSRC;         // [27][NSRC]
 
   const int tid = threadIdx.x;
-  const bool is_src = tid < TL::NSRC;
+  const bool is_src = tid < NSRC;
   const int sy = tid / BZ, sz = tid - (tid / BZ) * BZ;
-  const bool is_dst = tid < TL::NDST;
+  const bool is_dst = tid < NDST;
   const int ty = tid / TZ, tz = tid & (TZ - 1);
   const int dsrc = (ty + 1) * BZ + tz + 1;
   const long long N = a.N;
@@ -104,15 +101,9 @@ __global__ void __launch_bounds__(Tile<TY>::THREADS, 1) step_kernel(const StepAr
         if (PERIODIC) gx = ((gx % a.nx) + a.nx) % a.nx;
         else in = in && gx >= 0 && gx < a.nx;
         const T* g = cur + (in ? (long long)gx * plane + src_col : 0);
-        T* s = stage + (slot * 10) * TL::NSRC + tid;
+        T* s = stage + (slot * 10) * NSRC + tid;
 #pragma unroll
-        for (int k = 0; k < 10; ++k) {
-          if constexpr (sizeof(T) == 4) {
-            cp_async4(s + k * TL::NSRC, g + k * N, in ? 4 : 0);
-          } else {
-            s[k * TL::NSRC] = in ? g[k * N] : T(0);
-          }
-        }
+        for (int k = 0; k < 10; ++k) cp_async4(s + k * NSRC, g + k * N, in ? 4 : 0);
       }
       cp_async_commit();
     };
@@ -134,10 +125,10 @@ __global__ void __launch_bounds__(Tile<TY>::THREADS, 1) step_kernel(const StepAr
         R f[27];
         Mom3<R> m;
         if (in) {
-          const T* s = stage + ((it % NSTAGE) * 10) * TL::NSRC + tid;
+          const T* s = stage + ((it % NSTAGE) * 10) * NSRC + tid;
           R raw[10];
 #pragma unroll
-          for (int k = 0; k < 10; ++k) raw[k] = S::to_r(s[k * TL::NSRC]);
+          for (int k = 0; k < 10; ++k) raw[k] = S::to_r(s[k * NSRC]);
           m = decode3<S>(raw, a.sc);
         } else {
           // outside the domain: zero populations (f - w = -w), the reference's out-of-range rule
@@ -147,7 +138,7 @@ __global__ void __launch_bounds__(Tile<TY>::THREADS, 1) step_kernel(const StepAr
         }
         rebuild_all<R>(m, f);
 #pragma unroll
-        for (int d = 0; d < 27; ++d) mb[d * TL::NSRC + tid] = f[d];
+        for (int d = 0; d < 27; ++d) mb[d * NSRC + tid] = f[d];
       }
       __syncthreads();
       if (is_dst) {
@@ -160,7 +151,7 @@ __global__ void __launch_bounds__(Tile<TY>::THREADS, 1) step_kernel(const StepAr
           for (int yi = 0; yi < 3; ++yi)
 #pragma unroll
             for (int zi = 0; zi < 3; ++zi)
-              p[yi][zi] = mb[((xi * 3 + yi) * 3 + zi) * TL::NSRC + dsrc - (yi - 1) * BZ - (zi - 1)];
+              p[yi][zi] = mb[((xi * 3 + yi) * 3 + zi) * NSRC + dsrc - (yi - 1) * BZ - (zi - 1)];
           // c_x = -1 completes plane xs-1, 0 feeds plane xs, +1 starts plane xs+1
           if (xi == 0) accumulate_group<R>(acc_cur, p, -1);
           else if (xi == 1) accumulate_group<R>(acc_next, p, 0);
@@ -227,12 +218,6 @@ __global__ void __launch_bounds__(Tile<TY>::THREADS, 1) step_kernel(const StepAr
 }
 
 // ----------------------------------------------------------------------------- host side
-template <int TY, class S> size_t smem_bytes() {
-  using TL = Tile<TY>;
-  const size_t st = ((NSTAGE * 10 * TL::NSRC * sizeof(typename S::T) + 15) / 16) * 16;
-  return st + 27 * TL::NSRC * sizeof(typename S::R);
-}
-
 int num_sms() { return device_sms(); }
 
 // Work split: tiles x x-chunks. All CTAs march whole x ranges in step so that halo reloads
@@ -241,7 +226,7 @@ struct Plan {
   int tiles_y, tiles_z, n_tiles, chunks, chunk_len, n_items, grid;
 };
 
-template <int TY> Plan make_plan(int nx, int ny, int nz) {
+Plan make_plan(int nx, int ny, int nz) {
   Plan p;
   p.tiles_y = (ny + TY - 1) / TY;
   p.tiles_z = (nz + TZ - 1) / TZ;
@@ -285,9 +270,9 @@ void fill_diag(StepArgs& a, const hl_diag* diag) {
   a.health = diag->health;
 }
 
-template <int TY, class S, bool PERIODIC, bool FORCE, bool FLAGS, bool DIAG>
+template <bool PERIODIC, bool FORCE, bool FLAGS, bool DIAG>
 int launch_step(const hl_world3d* w, double vis_shear, const hl_diag* diag, cudaStream_t st) {
-  const Plan p = make_plan<TY>(w->nx, w->ny, w->nz);
+  const Plan p = make_plan(w->nx, w->ny, w->nz);
   StepArgs a{};
   a.cur = w->cur;
   a.post = w->post;
@@ -305,21 +290,19 @@ int launch_step(const hl_world3d* w, double vis_shear, const hl_diag* diag, cuda
   a.flag = w->flag;
   a.sc = make_scale(w->storage);
   if (DIAG) fill_diag(a, diag);
-  const size_t smem = smem_bytes<TY, S>();
-  auto kern = step_kernel<TY, S, PERIODIC, FORCE, FLAGS, DIAG>;
-  const int rc = set_smem_attr(reinterpret_cast<const void*>(kern), int(smem), "cudaFuncSetAttribute(d3q27 step)");
+  auto kern = step_kernel<PERIODIC, FORCE, FLAGS, DIAG>;
+  const int rc = set_smem_attr(reinterpret_cast<const void*>(kern), STEP_SMEM, "cudaFuncSetAttribute(d3q27 step)");
   if (rc != HL_OK) return rc;
-  kern<<<p.grid, Tile<TY>::THREADS, smem, st>>>(a);
+  kern<<<p.grid, STEP_THREADS, STEP_SMEM, st>>>(a);
   HL_LAUNCH_CHECK("d3q27 stream_collide launch");
   return HL_OK;
 }
 
-template <int TY, class S>
 int dispatch_step(const hl_world3d* w, double vis, const hl_diag* d, cudaStream_t st) {
   const bool P = w->periodic != 0, F = w->force != nullptr, G = w->flag != nullptr && !P,
              D = d != nullptr && d->scratch != nullptr;
 #define HL_D3_CASE(p, f, g, dg) \
-  if (P == p && F == f && G == g && D == dg) return launch_step<TY, S, p, f, g, dg>(w, vis, d, st);
+  if (P == p && F == f && G == g && D == dg) return launch_step<p, f, g, dg>(w, vis, d, st);
   HL_D3_CASE(true, false, false, false)
   HL_D3_CASE(true, false, false, true)
   HL_D3_CASE(true, true, false, false)
@@ -367,7 +350,7 @@ extern "C" int hl_d3q27_stream_collide(const hl_world3d* w, double vis_shear, co
   if (g_tune_d3_kernel != 1 && (plain ? d3::box_eligible(w) : d3::tma_eligible(w)))
     return d3::launch_step_tma(w, vis_shear, diag, st);
   switch (w->storage.dtype) {
-    case HL_F32: return d3::dispatch_step<16, StoreF32>(w, vis_shear, diag, st);
+    case HL_F32: return d3::dispatch_step(w, vis_shear, diag, st);
     case HL_F64: return d3::launch_sweep_f64(w, vis_shear, diag, st);
     default:
       set_error("d3q27: storage dtype %d not supported by this build", int(w->storage.dtype));
@@ -440,6 +423,6 @@ extern "C" int hl_d3q27_stream_collide_noalloc(const hl_world3d* w, double vis_s
   cudaError_t e = cudaMemsetAsync(scratch, 0, 16, st);
   if (e != cudaSuccess) return cuda_status(e, "hl_d3q27_stream_collide_noalloc: clear counter");
   hl_diag d{scratch, d3::kNoAllocScratchBytes, mass, health};
-  return w->storage.dtype == HL_F32 ? d3::dispatch_step<16, StoreF32>(w, vis_shear, &d, st)
+  return w->storage.dtype == HL_F32 ? d3::dispatch_step(w, vis_shear, &d, st)
                                     : d3::launch_sweep_f64(w, vis_shear, &d, st);
 }

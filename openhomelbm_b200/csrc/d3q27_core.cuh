@@ -1,4 +1,4 @@
-// Shared D3Q27 arithmetic of the stream-collide kernels (d3q27.cu, d3q27_tma.cu).
+// Shared D3Q27 arithmetic of the stream-collide kernels (d3q27.cu, d3q27_sweep.cuh, d3q27_mailbox.cu).
 #pragma once
 
 #include "hl_common.cuh"

@@ -1,5 +1,5 @@
 // D3Q27 arithmetic on cell pairs (P2 lanes = two consecutive x planes of one column), for
-// the TMA kernel (d3q27_tma.cu). Same mathematics as d3q27_core.cuh (the reference's
+// the 16-bit storages' kernel (d3q27_mailbox.cu). Same mathematics as d3q27_core.cuh (the reference's
 // mlCalEquilibrium3D_s rebuild, envs/lbm3d/lbm_func_3d.py:224-251, and the regularised
 // collision, 564-604), arranged so that constants enter through a few loop-invariant pairs
 // and every other operation is one packed instruction for both cells. The rearrangements

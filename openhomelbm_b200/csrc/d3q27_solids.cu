@@ -1,7 +1,7 @@
 // Immersed triangle-mesh solids of the D3Q27 step (sm_100a): the near-solid part of
 // stream_and_collide_3d (envs/lbm3d/lbm_func_3d.py:364-604).
 //
-// The stream-collide kernels (d3q27.cu, d3q27_tma.cu) update every fluid cell as if no solid
+// The stream-collide kernels (d3q27.cu, d3q27_sweep.cuh, d3q27_mailbox.cu) update every fluid cell as if no solid
 // existed. This file then recomputes the narrow band, the fluid cells within
 // bound_radius + 2 of a solid (387-393), with the reference's per-link logic:
 //   * the link's backward ray cell -> cell - c_i is cast against every solid near the cell

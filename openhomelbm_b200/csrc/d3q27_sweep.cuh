@@ -1,6 +1,6 @@
-// D3Q27 stream-collide by directional sweeps (sm_100a): the kernel behind both launchers,
-// d3q27_tma.cu (tiles staged by tensor copies) and d3q27.cu (any size and binary64, staged by
-// 4- or 8-byte asynchronous copies). It replaces stream_and_collide_3d for plain links
+// D3Q27 stream-collide by directional sweeps (sm_100a), binary32 and binary64 storage: the kernel behind
+// d3q27_tma.cu, staged by tensor copies, or for binary64 rows that those cannot take by 8-byte
+// asynchronous copies. It replaces stream_and_collide_3d for plain links
 // (envs/lbm3d/lbm_func_3d.py:364-604).
 //
 // The population that a cell sends along c is w_c (1 + g(c)) with, per source cell,
@@ -16,7 +16,7 @@
 // keeping 18 values of total order <= 2. No population is formed and none is exchanged:
 //   y: a lane holds two rows and reads the four source rows that feed them from shared memory;
 //   z: neighbouring lanes exchange 9 words per row and direction by warp shuffles; the columns
-//      beside the tile come from a helper warp that sweeps them along y ahead of the others;
+//      beside the tile are swept along y by the first lanes of each warp, for the warp's own rows;
 //   x: the block marches along x, and 15 values per cell wait in registers.
 // About 220 packed operations per pair of cells where forming, clamping and exchanging the
 // populations takes about 190 and 54 clamps, but no mailbox in shared memory (24 words
@@ -26,17 +26,15 @@
 // and 1 + 3q + 6 q^2 >= 5/8, so no population of a cell is negative while
 //     2 |u|^2 + 3/2 |Q:N| <= 5/8,   |u|^2 <= 3 U^2,  |Q:N| <= 8 n   (U, n: largest components),
 // which holds for any flow in the method's range (U up to 0.3). Each lane tracks the largest
-// components of the rows it reads, NaN included. The 16-bit storages hold N; plain storage holds S,
-// for which the same argument with 1 + 3q + 9/2 q^2 >= 1/2 gives 9/2 U^2 + 12 s <= 1/2 (U up to 0.17),
-// and where that fails the warp looks at N itself. Where the bound (with room to spare) fails in a
+// components of the rows it reads, NaN included. What is stored is S, for which the same argument with
+// 1 + 3q + 9/2 q^2 >= 1/2 gives 9/2 U^2 + 12 s <= 1/2 (U up to 0.17), and where that fails the warp looks
+// at N itself. Where the bound (with room to spare) fails in a
 // warp's rows, that warp computes the plane from clamped populations (clamped_sums), with the
 // reference's rule for every cell and NaN clamped to f = 0 as fmaxf does: the same step at about a
 // third of the rate (256^3 binary32 with U = 0.4 throughout).
 #pragma once
 
 #include <cuda.h>
-
-#include <type_traits>
 
 #include "d3q27_core.cuh"
 #include "d3q27_pair.cuh"
@@ -71,7 +69,7 @@ template <class R> constexpr int tile_y() { return CW * RPT * 32 / Lanes<R>::SEG
 // each for the tensor copies (WZ = 16 bytes of elements, the narrowest box), single elements for
 // the asynchronous copies. A periodic tile at the end of y has its outermost row wrap around: the
 // box leaves that row zero and its cells come as boxes of their own, [low, high row][10][32] and
-// [low, high row][side][10][WZ], which the helper warp moves into place.
+// [low, high row][side][10][WZ], which the warp that reads that row moves into place.
 template <class S, bool TMA, bool PERIODIC> struct Geo {
   using T = typename S::T;
   using R = typename S::R;
@@ -93,7 +91,7 @@ template <class S, bool TMA, bool PERIODIC> struct Geo {
   // columns for the latter
   static constexpr int WR = RPT * 32 / Lanes<R>::SEG, HS = WR + 2, HE = 12;
   static constexpr int HALO_B = CW * 2 * HS * HE * int(sizeof(R));
-  static_assert((ROWS + CW - 1) / CW <= 5, "rounds of element_row");
+  static_assert(TMA || (ROWS + CW - 1) / CW <= 3, "rounds of element_row");
   static_assert(!TMA || ROWS_B % 128 == 0, "tensor copies land on 128-byte boundaries");
 };
 template <class G, int NST> constexpr int smem_bytes() {
@@ -206,10 +204,9 @@ template <> struct Range<float> {
     for (int k = 4; k < 10; ++k) s = max3_abs(s, m[k].x(), m[k].y());
   }
   // true where some population may be negative (see the head of the file): s holds the largest
-  // component of S, or of N (N: the last argument; the reduced storages hold u / su and N / ss)
-  template <bool ENC> __device__ __forceinline__ bool clamps(const Scale& sc, bool n = ENC) const {
-    const float U = ENC ? u * sc.u : u, q = ENC ? s * sc.s : s;
-    return !((n ? fmaf(6.f * U, U, 12.f * q) <= 0.6f : fmaf(4.5f * U, U, 12.f * q) <= 0.45f) && d <= 1.f);
+  // component of S, or of N if n
+  __device__ __forceinline__ bool clamps(bool n) const {
+    return !((n ? fmaf(6.f * u, u, 12.f * s) <= 0.6f : fmaf(4.5f * u, u, 12.f * s) <= 0.45f) && d <= 1.f);
   }
 };
 template <> struct Range<double> {
@@ -222,7 +219,7 @@ template <> struct Range<double> {
 #pragma unroll
     for (int k = 4; k < 10; ++k) s = max(s, hi(m[k]));
   }
-  template <bool ENC> __device__ __forceinline__ bool clamps(const Scale&, bool n = ENC) const {
+  __device__ __forceinline__ bool clamps(bool n) const {
     // the largest value with this high word: NaN for the high words of infinity and of every NaN
     const double U = __hiloint2double(int(u), -1), q = __hiloint2double(int(s), -1);
     return !((n ? 6.0 * U * U + 12.0 * q <= 0.6 : 4.5 * U * U + 12.0 * q <= 0.45) && d < 0x40000000u);  // 0 <= rho < 2
@@ -258,53 +255,20 @@ template <class V> struct Coef {
   V A, Bx, By, Bz, Cxx, Cyy, Czz, Dxy, Dxz, Dyz;
 };
 
-// Loop-invariant factors of the reduced storages' decode: u = su raw, S - u u = ss raw, folded
-// into B_a = (3 su rho) raw_a, D_ab = B_a (4 su raw_b) + (3 ss rho) raw_ab and C_aa = D_aa / 2.
-template <class V> struct Decode {
-  V su3, su4, su2, ss3, ss15;
-};
-template <class V, class R> __device__ __forceinline__ Decode<V> make_decode(const Scale& sc) {
-  Decode<V> d;
-  d.su3 = bcast(V(), R(3) * R(sc.u));
-  d.su4 = bcast(V(), R(4) * R(sc.u));
-  d.su2 = bcast(V(), R(2) * R(sc.u));
-  d.ss3 = bcast(V(), R(3) * R(sc.s));
-  d.ss15 = bcast(V(), R(1.5) * R(sc.s));
-  return d;
-}
-
-template <class S, class V, class R>
-__device__ __forceinline__ Coef<V> coefficients(const V raw[10], const Decode<V>& dc, Range<R>& rg) {
+template <class V, class R> __device__ __forceinline__ Coef<V> coefficients(const V raw[10], Range<R>& rg) {
   Coef<V> c;
-  V drho;
-  if constexpr (S::kEncoded) {
-    drho = raw[0];
-    const V rho = raw[0] + V(1.0);
-    const V r3u = rho * dc.su3, r3s = rho * dc.ss3, r15s = rho * dc.ss15;
-    c.Bx = r3u * raw[1];
-    c.By = r3u * raw[2];
-    c.Bz = r3u * raw[3];
-    const V qy = raw[2] * dc.su4, qz = raw[3] * dc.su4;
-    c.Cxx = c.Bx * V(raw[1] * dc.su2) + r15s * raw[4];
-    c.Cyy = c.By * V(raw[2] * dc.su2) + r15s * raw[5];
-    c.Czz = c.Bz * V(raw[3] * dc.su2) + r15s * raw[6];
-    c.Dxy = c.Bx * qy + r3s * raw[7];
-    c.Dxz = c.Bx * qz + r3s * raw[8];
-    c.Dyz = c.By * qz + r3s * raw[9];
-  } else {
-    drho = raw[0] - V(1.0);
-    const V r3 = raw[0] * V(3.0), r15 = raw[0] * V(1.5);
-    const V vx = raw[1] * V(3.0), vy = raw[2] * V(3.0), vz = raw[3] * V(3.0);
-    c.Bx = r3 * raw[1];
-    c.By = r3 * raw[2];
-    c.Bz = r3 * raw[3];
-    c.Cxx = r15 * V(vx * raw[1] + raw[4]);
-    c.Cyy = r15 * V(vy * raw[2] + raw[5]);
-    c.Czz = r15 * V(vz * raw[3] + raw[6]);
-    c.Dxy = r3 * V(vx * raw[2] + raw[7]);
-    c.Dxz = r3 * V(vx * raw[3] + raw[8]);
-    c.Dyz = r3 * V(vy * raw[3] + raw[9]);
-  }
+  const V drho = raw[0] - V(1.0);
+  const V r3 = raw[0] * V(3.0), r15 = raw[0] * V(1.5);
+  const V vx = raw[1] * V(3.0), vy = raw[2] * V(3.0), vz = raw[3] * V(3.0);
+  c.Bx = r3 * raw[1];
+  c.By = r3 * raw[2];
+  c.Bz = r3 * raw[3];
+  c.Cxx = r15 * V(vx * raw[1] + raw[4]);
+  c.Cyy = r15 * V(vy * raw[2] + raw[5]);
+  c.Czz = r15 * V(vz * raw[3] + raw[6]);
+  c.Dxy = r3 * V(vx * raw[2] + raw[7]);
+  c.Dxz = r3 * V(vx * raw[3] + raw[8]);
+  c.Dyz = r3 * V(vy * raw[3] + raw[9]);
   rg.add(drho, raw);
   const V tr = (c.Cxx + c.Cyy) + c.Czz;
   c.A = tr * V(-1.0 / 3.0) + drho;
@@ -420,29 +384,18 @@ template <class G> struct Stage {
   }
 };
 
-template <class S> __device__ __forceinline__ P2 load_vec(P2, const typename S::T* p) {
-  if constexpr (sizeof(typename S::T) == 4) {
-    return P2(*reinterpret_cast<const float2*>(p));
-  } else {
-    const unsigned v = *reinterpret_cast<const unsigned*>(p);
-    if constexpr (std::is_same<S, StoreF16>::value) {
-      return P2(__half22float2(*reinterpret_cast<const __half2*>(&v)));
-    } else {
-      return P2(__uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u));
-    }
-  }
-}
-template <class S> __device__ __forceinline__ double load_vec(double, const typename S::T* p) { return *p; }
+__device__ __forceinline__ P2 load_vec(P2, const float* p) { return P2(*reinterpret_cast<const float2*>(p)); }
+__device__ __forceinline__ double load_vec(double, const double* p) { return *p; }
 
 template <class V> struct Ten {
   V v[10];
   __device__ __forceinline__ V& operator[](int k) { return v[k]; }
 };
 
-// Plain storage: whether the cells that feed a lane's rows may send a negative population, by
+// Whether the cells that feed a lane's rows may send a negative population, by
 // N = S - u u (the source rows from `row` - 1 on, and the lane's halo cell).
 template <class S, class V, class G>
-__device__ __forceinline__ bool may_clamp(const Stage<G>& st, int row, int z, int hrow, int hside, const Scale& sc) {
+__device__ __forceinline__ bool may_clamp(const Stage<G>& st, int row, int z, int hrow, int hside) {
   using R = typename S::R;
   Range<R> rg;
   auto look = [&](auto raw) {
@@ -461,7 +414,7 @@ __device__ __forceinline__ bool may_clamp(const Stage<G>& st, int row, int z, in
     const typename S::T* src = st.row(row + dr, z);
     Ten<V> raw;
 #pragma unroll
-    for (int k = 0; k < 10; ++k) raw[k] = load_vec<S>(V(), src + k * G::MS);
+    for (int k = 0; k < 10; ++k) raw[k] = load_vec(V(), src + k * G::MS);
     look(raw);
   }
   const typename S::T* src = st.column(hrow, hside);
@@ -469,16 +422,14 @@ __device__ __forceinline__ bool may_clamp(const Stage<G>& st, int row, int z, in
 #pragma unroll
   for (int k = 0; k < 10; ++k) raw[k] = S::to_r(src[k * G::CS]);
   look(raw);
-  return rg.template clamps<false>(sc, true);
+  return rg.clamps(true);
 }
 
 // One destination row's sums from its neighbours' clamped populations (f >= 0 is g >= -1), every
-// source cell read from the stage. zero: what lies outside the domain and must read as the zero
-// cell (bits 0..2 the rows -1, 0, +1 from this one, bits 3 and 4 the columns -1 and 32); only the
-// encoded storages need it, where a zero-filled cell is rho = 1.
+// source cell read from the stage. What lies outside a walled domain was staged as zeros, which are the
+// cell of zero populations that the reference's out-of-range rule asks for.
 template <class S, class V, class G>
-__device__ __forceinline__ void clamped_sums(const Stage<G>& st, int row, int z, const Decode<V>& dc, unsigned zero,
-                                             Sums<V>& s) {
+__device__ __forceinline__ void clamped_sums(const Stage<G>& st, int row, int z, Sums<V>& s) {
   using R = typename S::R;
   constexpr int NZ = Lanes<R>::NZ;
 #pragma unroll
@@ -495,7 +446,6 @@ __device__ __forceinline__ void clamped_sums(const Stage<G>& st, int row, int z,
       const int stride = col ? G::CS : G::MS;
 #pragma unroll
       for (int k = 0; k < 10; ++k) v[e][k] = S::to_r(p[k * stride]);
-      if ((zero >> (dy + 1)) & 1u || (zc < 0 && (zero & 8u)) || (zc >= TZ && (zero & 16u))) v[e][0] = R(-1);
     }
     V raw[10];
 #pragma unroll
@@ -504,7 +454,7 @@ __device__ __forceinline__ void clamped_sums(const Stage<G>& st, int row, int z,
       else raw[k] = v[0][k];
     }
     Range<R> unused;
-    const Coef<V> c = coefficients<S, V, R>(raw, dc, unused);
+    const Coef<V> c = coefficients<V, R>(raw, unused);
     const V cy = bcast(V(), R(-dy)), cz = bcast(V(), R(-dz));
     const V cy2 = bcast(V(), R(dy * dy)), cz2 = bcast(V(), R(dz * dz)), cyz = bcast(V(), R(dy * dz));
     V p = c.A, q = c.Bx;  // no products by zero: a NaN must stay out of the directions it is not in
@@ -562,26 +512,17 @@ template <class V> __device__ __forceinline__ void sweep_x(Carry<V>& c, const Su
   }
 }
 
-// Loop-invariant factors of the collision and of the encode.
+// Loop-invariant factors of the collision: omega, 1 - omega, (1 - omega) / 3.
 template <class V> struct Collide {
-  V om, o1, o13, iu;  // binary32/64: omega, 1 - omega, (1 - omega) / 3; encoded: see make_collide
+  V om, o1, o13;
 };
-template <class S, class V> __device__ __forceinline__ Collide<V> make_collide(double vis, const Scale& sc) {
-  using R = typename S::R;
+template <class V, class R> __device__ __forceinline__ Collide<V> make_collide(double vis) {
   const R omega = R(1) / (R(vis) * R(3) + R(0.5));
-  Collide<V> k;
   const R o1 = R(1) - omega;
-  if constexpr (S::kEncoded) {  // the stored S - u u, scaled: omega - 1 in place of omega
-    k.om = bcast(V(), -o1 * R(sc.inv_s));
-    k.o1 = bcast(V(), o1 * R(sc.inv_s));
-    k.o13 = bcast(V(), o1 * R(1.0 / 3.0) * R(sc.inv_s));
-    k.iu = bcast(V(), R(sc.inv_u));
-  } else {
-    k.om = bcast(V(), omega);
-    k.o1 = bcast(V(), o1);
-    k.o13 = bcast(V(), o1 * R(1.0 / 3.0));
-    k.iu = V(1.0);
-  }
+  Collide<V> k;
+  k.om = bcast(V(), omega);
+  k.o1 = bcast(V(), o1);
+  k.o13 = bcast(V(), o1 * R(1.0 / 3.0));
   return k;
 }
 
@@ -589,12 +530,9 @@ template <class S, class V> __device__ __forceinline__ Collide<V> make_collide(d
 // planes. With P = sums - delta/3 and R_a = rho u_a^2 the reference's
 //   X_aa = (1-omega)(P_aa - tr P/3 + tr R/3) + omega R_a + F_a u_a,  S_aa = X_aa / rho
 // is S_aa = omega u_a^2 + (1-omega)(P_aa/rho - tr P/(3 rho) + u.u/3) + F_a u_a / rho, so only P is
-// divided by rho. The encoded storages keep S - u' u' (u' = u + F/(2 rho), the stored velocity):
-// the force terms of S and of u' u' cancel but for -(F_a F_b)/(4 rho^2).
-template <class S, bool FORCE, class V>
-__device__ __forceinline__ void collide_raw(const Totals<V>& t, const V F[3], const Collide<V>& k, const Scale& sc,
-                                              V raw[10], V& rho_out) {
-  using R = typename S::R;
+// divided by rho.
+template <class R, bool FORCE, class V>
+__device__ __forceinline__ void collide_raw(const Totals<V>& t, const V F[3], const Collide<V>& k, V raw[10]) {
   // -216 exactly where no population arrives: drho -1 and rho 0, which the health count and a step of
   // such a cell need, if the product is rounded before the sum (fused, rho is the constant's error)
   const V drho = mul_rn(t.z[0], R(1.0 / 216.0));
@@ -620,40 +558,22 @@ __device__ __forceinline__ void collide_raw(const Totals<V>& t, const V F[3], co
   V s[6] = {V(k.om * xx + (oi * t.txx + base)), V(k.om * yy + (oi * t.z[3] + base)), V(k.om * zz + (oi * t.z[4] + base)),
             V(k.om * V(ux * uy) + oi * t.mxy), V(k.om * V(ux * uz) + oi * t.mxz), V(k.om * V(uy * uz) + oi * t.z[5])};
   if (FORCE) {
-    if constexpr (S::kEncoded) {
-      const V is = bcast(V(), R(sc.inv_s));
-      const V gx = fx * is, gy = fy * is, gz = fz * is;
-      s[0] = s[0] - gx * fx;
-      s[1] = s[1] - gy * fy;
-      s[2] = s[2] - gz * fz;
-      s[3] = s[3] - gx * fy;
-      s[4] = s[4] - gx * fz;
-      s[5] = s[5] - gy * fz;
-    } else {
-      s[0] = (fx + fx) * ux + s[0];
-      s[1] = (fy + fy) * uy + s[1];
-      s[2] = (fz + fz) * uz + s[2];
-      s[3] = fx * uy + (fy * ux + s[3]);
-      s[4] = fx * uz + (fz * ux + s[4]);
-      s[5] = fy * uz + (fz * uy + s[5]);
-    }
+    s[0] = (fx + fx) * ux + s[0];
+    s[1] = (fy + fy) * uy + s[1];
+    s[2] = (fz + fz) * uz + s[2];
+    s[3] = fx * uy + (fy * ux + s[3]);
+    s[4] = fx * uz + (fz * ux + s[4]);
+    s[5] = fy * uz + (fz * uy + s[5]);
     ux = ux + fx;
     uy = uy + fy;
     uz = uz + fz;
   }
-  raw[0] = S::kEncoded ? drho : rho;
-  if constexpr (S::kEncoded) {
-    raw[1] = ux * k.iu;
-    raw[2] = uy * k.iu;
-    raw[3] = uz * k.iu;
-  } else {
-    raw[1] = ux;
-    raw[2] = uy;
-    raw[3] = uz;
-  }
+  raw[0] = rho;
+  raw[1] = ux;
+  raw[2] = uy;
+  raw[3] = uz;
 #pragma unroll
   for (int i = 0; i < 6; ++i) raw[4 + i] = s[i];
-  rho_out = rho;
 }
 
 // ---------------------------------------------------------------- the kernel
@@ -673,10 +593,7 @@ __global__ void __launch_bounds__(THREADS, MINB)
   using G = Geo<S, TMA, PERIODIC>;
   constexpr int NZ = LN::NZ, SEG = LN::SEG, TY = G::TY;
   // Cells outside a walled domain must read as the zero cell (zero populations: the reference's
-  // out-of-range rule). Staging zero-fills them, which IS the zero cell of plain storage; the
-  // encoded storages hold rho - 1 and need a select where an outside cell can feed a stored one:
-  // with a flag array, where a border cell may be fluid. Without one only interior cells are stored.
-  constexpr bool SEL = S::kEncoded && FLAGS && !PERIODIC;
+  // out-of-range rule): staging zero-fills them.
   extern __shared__ __align__(128) unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -798,8 +715,8 @@ __global__ void __launch_bounds__(THREADS, MINB)
       }
     }
   };
-  // Asynchronous copies: the warps take the tile's rows in turn, a lane per column, and 36 (binary64:
-  // 20) x 3 threads the halo columns' cells, every third moment each.
+  // Asynchronous copies: the warps take the tile's rows in turn, a lane per column, and 20 x 3 threads the
+  // halo columns' cells, every third moment each.
   constexpr int COLS = 2 * G::ROWS;
   const int e_cell = tid % COLS, e_k0 = tid / COLS;  // halo cell (side, row) and first moment
   const int e_side = e_cell / G::ROWS, e_row = e_cell % G::ROWS;
@@ -883,9 +800,7 @@ __global__ void __launch_bounds__(THREADS, MINB)
   const int zt = l * NZ;
   // lanes 0 .. 2 HS - 1 sweep the halo columns: column lane / HS, source row rb - 1 + lane % HS
   const int hside = lane >= G::HS ? 1 : 0, hrow = rb - 1 + (lane < 2 * G::HS ? lane - hside * G::HS : 0);
-  const Decode<V> dc = make_decode<V, R>(a.sc);
-  const Decode<R> dh = make_decode<R, R>(a.sc);
-  const Collide<V> kc = make_collide<S, V>(a.vis_shear, a.sc);
+  const Collide<V> kc = make_collide<V, R>(a.vis_shear);
   long long N = a.N;
   int nx = a.nx, ny = a.ny, nz = a.nz;
   T* post = static_cast<T*>(a.post);
@@ -963,12 +878,8 @@ __global__ void __launch_bounds__(THREADS, MINB)
         const T* src = st.row(r0 + dr, zt);
         V raw[10];
 #pragma unroll
-        for (int k = 0; k < 10; ++k) raw[k] = load_vec<S>(V(), src + k * G::MS);
-        if (SEL) {
-          const int gy = y0 + r0 + dr;
-          if (!(xs >= 0 && xs < nx && gy >= 0 && gy < ny)) raw[0] = V(-1.0);
-        }
-        return coefficients<S, V, R>(raw, dc, rg);
+        for (int k = 0; k < 10; ++k) raw[k] = load_vec(V(), src + k * G::MS);
+        return coefficients<V, R>(raw, rg);
       };
       element_row(1);
       V p[RPT][6], o[RPT][6], m[RPT][6];
@@ -989,11 +900,7 @@ __global__ void __launch_bounds__(THREADS, MINB)
         R raw[10];
 #pragma unroll
         for (int k = 0; k < 10; ++k) raw[k] = S::to_r(src[k * G::CS]);
-        if (SEL) {
-          const int gy = y0 + hrow, gz = hside ? z0 + TZ : z0 - 1;
-          if (!(xs >= 0 && xs < nx && gy >= 0 && gy < ny && gz >= 0 && gz < nz)) raw[0] = R(-1);
-        }
-        const Coef<R> c = coefficients<S, R, R>(raw, dh, rg);
+        const Coef<R> c = coefficients<R, R>(raw, rg);
         R p[6], o[6], m[6], y[3][6], w[9];
         along_y<1>(c, p);
         along_y<0>(c, o);
@@ -1016,26 +923,12 @@ __global__ void __launch_bounds__(THREADS, MINB)
         __syncwarp();
       }
       // One vote for the lane's rows, and both rows in one stretch of code: their chains overlap.
-      bool neg = __any_sync(FULL, rg.template clamps<S::kEncoded>(a.sc));
-      if constexpr (!S::kEncoded) {
-        if (neg) neg = __any_sync(FULL, may_clamp<S, V, G>(st, r0, zt, hrow, hside, a.sc));
-      }
+      bool neg = __any_sync(FULL, rg.clamps(false));
+      if (neg) neg = __any_sync(FULL, may_clamp<S, V, G>(st, r0, zt, hrow, hside));
       Sums<V> sums[RPT];
       if (neg) {
 #pragma unroll
-        for (int r = 0; r < RPT; ++r) {
-          unsigned zero = 0u;
-          if (SEL) {
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-              const int gy = y0 + r0 + r + k - 1;
-              if (!(xs >= 0 && xs < nx && gy >= 0 && gy < ny)) zero |= 1u << k;
-            }
-            if (z0 == 0) zero |= 8u;
-            if (z0 + TZ >= nz) zero |= 16u;
-          }
-          clamped_sums<S, V, G>(st, r0 + r, zt, dc, zero, sums[r]);
-        }
+        for (int r = 0; r < RPT; ++r) clamped_sums<S, V, G>(st, r0 + r, zt, sums[r]);
       } else {
 #pragma unroll
         for (int r = 0; r < RPT; ++r) {
@@ -1047,58 +940,35 @@ __global__ void __launch_bounds__(THREADS, MINB)
         }
       }
       stage_boxes(q & (CW - 1));
-      element_row(3);
-      element_row(4);
       Totals<V> tot[RPT];
 #pragma unroll
       for (int r = 0; r < RPT; ++r) sweep_x(carry[r], sums[r], tot[r]);
       if (store) {
-        V raws[RPT][10], rhos[RPT];
+        V raws[RPT][10];
 #pragma unroll
-        for (int r = 0; r < RPT; ++r) collide_raw<S, FORCE>(tot[r], F[r], kc, a.sc, raws[r], rhos[r]);
+        for (int r = 0; r < RPT; ++r) collide_raw<R, FORCE>(tot[r], F[r], kc, raws[r]);
 #pragma unroll
         for (int r = 0; r < RPT; ++r) {
           const V(&raw)[10] = raws[r];
-          const V rho = rhos[r];
+          const V rho = raw[0];
           const int y = y0 + r0 + r;
           const unsigned cell = unsigned(y) * unsigned(nz) + unsigned(dz);  // within the plane
           // 32-bit cell indices reach every plane of 4- and 8-byte storage that fits a GPU
-          using I = typename std::conditional<sizeof(T) == 2, long long, unsigned>::type;
-          const I ci = I(d) * I(plane) + I(cell);
+          const unsigned ci = unsigned(d) * unsigned(plane) + cell;
           auto pk = [&](int k) { return BATCH ? post + k * N : static_cast<T*>(a.post_k[k]); };
           if constexpr (NZ == 2) {
             const bool both = on[r][0] && on[r][1];
-            if constexpr (S::kEncoded) {
-              const unsigned cs0 = unsigned(ci) * 0x9e3779b9u, cs1 = cs0 + 0x9e3779b9u;
-              unsigned v[10];
+            if (both) {
 #pragma unroll
-              for (int k = 0; k < 10; ++k) v[k] = S::round2(raw[k].y(), raw[k].x(), cs1, cs0, unsigned(k));
-              if (both) {
-#pragma unroll
-                for (int k = 0; k < 10; ++k) *reinterpret_cast<unsigned*>(pk(k) + ci) = v[k];
-              } else {
-                if (on[r][0]) {
-#pragma unroll
-                  for (int k = 0; k < 10; ++k) pk(k)[ci] = S::lo(v[k]);
-                }
-                if (on[r][1]) {
-#pragma unroll
-                  for (int k = 0; k < 10; ++k) (pk(k) + ci)[1] = S::hi(v[k]);
-                }
-              }
+              for (int k = 0; k < 10; ++k) *reinterpret_cast<float2*>(pk(k) + ci) = raw[k].v;
             } else {
-              if (both) {
+              if (on[r][0]) {
 #pragma unroll
-                for (int k = 0; k < 10; ++k) *reinterpret_cast<float2*>(pk(k) + ci) = raw[k].v;
-              } else {
-                if (on[r][0]) {
+                for (int k = 0; k < 10; ++k) pk(k)[ci] = raw[k].x();
+              }
+              if (on[r][1]) {
 #pragma unroll
-                  for (int k = 0; k < 10; ++k) pk(k)[ci] = raw[k].x();
-                }
-                if (on[r][1]) {
-#pragma unroll
-                  for (int k = 0; k < 10; ++k) (pk(k) + ci)[1] = raw[k].y();
-                }
+                for (int k = 0; k < 10; ++k) (pk(k) + ci)[1] = raw[k].y();
               }
             }
             if (DIAG) {
@@ -1171,9 +1041,9 @@ __global__ void __launch_bounds__(THREADS, MINB)
 }
 
 // ---------------------------------------------------------------- host side
-// Blocks resident per SM: two of 160 threads. binary32 holds two blocks of three staged planes in
-// shared memory (92 KB each); the 16-bit storages have room for four planes.
-template <class S, bool TMA> constexpr int stages() { return !TMA || sizeof(typename S::T) == 2 ? 4 : 3; }
+// Blocks resident per SM: two of 128 threads, each with three staged planes in shared memory (87 KB walled,
+// 98 KB periodic in binary32); four where 8-byte copies need one plane more.
+template <class S, bool TMA> constexpr int stages() { return TMA ? 3 : 4; }
 constexpr int BLOCKS_PER_SM = 2;
 
 // Work split: tiles x x-chunks, equal chunks dealt round-robin, so that all blocks march x together
@@ -1217,7 +1087,6 @@ int launch(const hl_world3d* w, double vis, const hl_diag* diag, const Maps& map
   a.vis_shear = vis;
   a.force = w->force;
   a.flag = w->flag;
-  a.sc = make_scale(w->storage);
   for (int k = 0; k < 10; ++k) {
     a.cur_k[k] = static_cast<const typename S::T*>(w->cur) + k * a.N;
     a.post_k[k] = static_cast<typename S::T*>(w->post) + k * a.N;
@@ -1260,5 +1129,6 @@ int dispatch(const hl_world3d* w, double vis, const hl_diag* d, const Maps& maps
 }
 
 }  // namespace sw
+
 }  // namespace d3
 }  // namespace hl

@@ -1,12 +1,13 @@
-// D3Q27 stream-collide over tiles staged by the tensor memory accelerator (sm_100a): the sweep
-// kernel of d3q27_sweep.cuh for domains of whole tiles (ny a multiple of 16, nz of 32) in binary32,
-// binary16 or bfloat16 storage, alone or many domains in one launch.
+// Launchers of the D3Q27 sweep kernel (d3q27_sweep.cuh) for domains whose rows are multiples of 16 bytes
+// (walled tiles may reach past the domain; periodic domains are whole tiles), staged by the tensor memory
+// accelerator: binary32, alone or many domains in one launch, and binary64. The
+// 16-bit storages go on to d3q27_mailbox.cu with tensor maps from here.
 //
-// Staging: per plane a warp issues a box copy of each of the tile's 18 rows (32 z x 10 moments),
-// one 16-byte wide box for the column before and after the tile and four for its corners, every
-// box with its own coordinates, so that periodic wrap-around of the halo is just a coordinate, and
-// boxes outside a walled domain are zero-filled by the copy. Completion is tracked by one mbarrier
-// per stage with bounded waits. No multicast: every block loads its own boxes.
+// Staging: per plane one thread issues a box copy of the tile's rows with the one beyond either end and
+// a 16-byte wide box for the column before and after the tile. Periodic wrap-around along x and z is a
+// coordinate; a row beyond y's ends comes as boxes of its own. Boxes outside a walled domain are
+// zero-filled by the copy. Completion is tracked by one mbarrier per stage with bounded waits. No
+// multicast: every block loads its own boxes.
 
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -102,14 +103,12 @@ std::mutex g_batch_mu;
 std::map<const void*, std::pair<int, int>> g_batches;
 
 template <class S>
-int launch_batch(const BatchDomain* doms, int n_doms, int n_items, double vis, const hl_storage& storage, int parity,
-                 int* status, cudaStream_t st) {
+int launch_batch(const BatchDomain* doms, int n_doms, int n_items, double vis, int parity, int* status, cudaStream_t st) {
   using G = sw::Geo<S, true, false>;
   constexpr int NST = sw::stages<S, true>(), SMEM = sw::smem_bytes<G, NST>();
   StepArgs a{};
   a.n_items = n_items;
   a.vis_shear = vis;
-  a.sc = make_scale(storage);
   a.status = status;
   Maps maps;
   std::memset(&maps, 0, sizeof(maps));
@@ -248,7 +247,7 @@ extern "C" int hl_d3q27_stream_collide_batch(const void* desc, int n_domains, in
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const auto* doms = static_cast<const d3::tma::BatchDomain*>(desc);
   switch (storage->dtype) {
-    case HL_F32: return d3::tma::launch_batch<StoreF32>(doms, n_domains, n_items, vis_shear, *storage, parity, status, st);
+    case HL_F32: return d3::tma::launch_batch<StoreF32>(doms, n_domains, n_items, vis_shear, parity, status, st);
     case HL_F16:
     case HL_BF16: return d3::launch_mailbox_batch(doms, n_domains, n_items, vis_shear, *storage, parity, status, st);
     default: break;

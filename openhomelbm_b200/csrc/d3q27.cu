@@ -38,7 +38,6 @@
 #include <algorithm>
 #include <cstdio>
 #include <cstdlib>
-#include <cstring>
 
 #include "d3q27_sweep.cuh"
 
@@ -320,13 +319,6 @@ int dispatch_step(const hl_world3d* w, double vis, const hl_diag* d, cudaStream_
   return HL_ERR_UNSUPPORTED;
 }
 
-// binary64 with rows that are no multiple of 16 bytes: the sweeps staged by 8-byte copies
-int launch_sweep_f64(const hl_world3d* w, double vis, const hl_diag* diag, cudaStream_t st) {
-  sw::Maps unused;
-  std::memset(&unused, 0, sizeof(unused));
-  return sw::dispatch<StoreF64, false>(w, vis, diag, unused, st);
-}
-
 }  // namespace d3
 }  // namespace hl
 
@@ -351,7 +343,7 @@ extern "C" int hl_d3q27_stream_collide(const hl_world3d* w, double vis_shear, co
     return d3::launch_step_tma(w, vis_shear, diag, st);
   switch (w->storage.dtype) {
     case HL_F32: return d3::dispatch_step(w, vis_shear, diag, st);
-    case HL_F64: return d3::launch_sweep_f64(w, vis_shear, diag, st);
+    case HL_F64: return d3::launch_sweep_f64(w, vis_shear, diag, nullptr, st);
     default:
       set_error("d3q27: storage dtype %d not supported by this build", int(w->storage.dtype));
       return HL_ERR_UNSUPPORTED;
@@ -424,5 +416,5 @@ extern "C" int hl_d3q27_stream_collide_noalloc(const hl_world3d* w, double vis_s
   if (e != cudaSuccess) return cuda_status(e, "hl_d3q27_stream_collide_noalloc: clear counter");
   hl_diag d{scratch, d3::kNoAllocScratchBytes, mass, health};
   return w->storage.dtype == HL_F32 ? d3::dispatch_step(w, vis_shear, &d, st)
-                                    : d3::launch_sweep_f64(w, vis_shear, &d, st);
+                                    : d3::launch_sweep_f64(w, vis_shear, &d, nullptr, st);
 }

@@ -1130,5 +1130,8 @@ int dispatch(const hl_world3d* w, double vis, const hl_diag* d, const Maps& maps
 
 }  // namespace sw
 
+// binary64 (d3q27_sweep_f64.cu): by tensor copies, or without maps by 8-byte copies
+int launch_sweep_f64(const hl_world3d* w, double vis_shear, const hl_diag* diag, const sw::Maps* maps, cudaStream_t st);
+
 }  // namespace d3
 }  // namespace hl

@@ -1,6 +1,6 @@
 // Launchers of the D3Q27 sweep kernel (d3q27_sweep.cuh) for domains whose rows are multiples of 16 bytes
 // (walled tiles may reach past the domain; periodic domains are whole tiles), staged by the tensor memory
-// accelerator: binary32, alone or many domains in one launch, and binary64. The
+// accelerator: binary32, alone or many domains in one launch, and binary64 (d3q27_sweep_f64.cu). The
 // 16-bit storages go on to d3q27_mailbox.cu with tensor maps from here.
 //
 // Staging: per plane one thread issues a box copy of the tile's rows with the one beyond either end and
@@ -152,7 +152,7 @@ int launch_step_tma(const hl_world3d* w, double vis, const hl_diag* diag, cudaSt
   if (mailbox) return launch_mailbox(w, vis, diag, maps, st);
   switch (dt) {
     case HL_F32: return sw::dispatch<StoreF32, true>(w, vis, diag, maps, st);
-    case HL_F64: return sw::dispatch<StoreF64, true>(w, vis, diag, maps, st);
+    case HL_F64: return launch_sweep_f64(w, vis, diag, &maps, st);
     default: break;
   }
   set_error("d3q27 (tma): dtype not supported");

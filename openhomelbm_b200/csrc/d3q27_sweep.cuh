@@ -170,9 +170,14 @@ __device__ __forceinline__ P2 reciprocal(P2 x) {
   return r0 * (P2(1.0) - x * r0) + r0;
 }
 __device__ __forceinline__ double reciprocal(double x) { return 1.0 / x; }
-// a * b, never fused into what uses it
-__device__ __forceinline__ P2 mul_rn(P2 a, float b) { return P2(__fmul_rn(a.x(), b), __fmul_rn(a.y(), b)); }
-__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+// z / 216 + 1, in one rounding
+__device__ __forceinline__ P2 plus_one(P2 z) { return z * P2(1.0 / 216.0) + P2(1.0); }
+__device__ __forceinline__ double plus_one(double z) { return __fma_rn(z, 1.0 / 216.0, 1.0); }
+// v, or `instead` where z is -216
+__device__ __forceinline__ P2 unless_empty(P2 z, P2 v, float instead) {
+  return P2(z.x() == -216.f ? instead : v.x(), z.y() == -216.f ? instead : v.y());
+}
+__device__ __forceinline__ double unless_empty(double z, double v, double instead) { return z == -216.0 ? instead : v; }
 __device__ __forceinline__ P2 bcast(P2, float v) { return P2(v, v); }
 __device__ __forceinline__ double bcast(double, double v) { return v; }
 __device__ __forceinline__ float bcast(float, float v) { return v; }
@@ -535,10 +540,11 @@ template <class V, class R> __device__ __forceinline__ Collide<V> make_collide(d
 // divided by rho.
 template <class R, bool FORCE, class V>
 __device__ __forceinline__ void collide_raw(const Totals<V>& t, const V F[3], const Collide<V>& k, V raw[10]) {
-  // -216 exactly where no population arrives: drho -1 and rho 0, which the health count and a step of
-  // such a cell need, if the product is rounded before the sum (fused, rho is the constant's error)
-  const V drho = mul_rn(t.z[0], R(1.0 / 216.0));
-  const V rho = drho + V(1.0);
+  // The sum is -216 exactly where no population arrives, in a cavity or beside cells that are NaN: density
+  // and velocity zero, which the health count and the steps of such a cell need (1 + z / 216 as one
+  // multiply-add is the constant's error). Divided by 1, not by 0: a binary64 division by zero is a slow
+  // one, and the lanes past the end of a domain are such cells.
+  const V rho = unless_empty(t.z[0], plus_one(t.z[0]), 1);
   const V inv = reciprocal(rho);
   const V i216 = inv * V(1.0 / 216.0);
   V ux = t.mx * i216, uy = t.z[1] * i216, uz = t.z[2] * i216;
@@ -570,7 +576,7 @@ __device__ __forceinline__ void collide_raw(const Totals<V>& t, const V F[3], co
     uy = uy + fy;
     uz = uz + fz;
   }
-  raw[0] = rho;
+  raw[0] = unless_empty(t.z[0], rho, 0);
   raw[1] = ux;
   raw[2] = uy;
   raw[3] = uz;

@@ -1056,7 +1056,9 @@ constexpr int BLOCKS_PER_SM = 2;
 
 // Work split: tiles x x-chunks, equal chunks dealt round-robin, so that all blocks march x together
 // and the halos of neighbouring tiles are L2 hits; x is split where that fills the SMs with less
-// waste than the two halo planes that each chunk reads on top.
+// waste than the two halo planes that each chunk reads on top. More than 64 chunks where they keep four
+// planes, for a long domain of few tiles: 1000 x 16 x 32 binary32 in 64 chunks 30.5 us, in 250 14.5 (the kernel
+// before: 27.4).
 inline void split_x(StepArgs& a, int ty) {
   a.tiles_y = (a.ny + ty - 1) / ty;
   a.tiles_z = (a.nz + TZ - 1) / TZ;
@@ -1065,9 +1067,10 @@ inline void split_x(StepArgs& a, int ty) {
   const int forced = g_tune_d3_chunks;
   int best_c = 1;
   double best = -1;
-  for (int c = 1; c <= 64 && c <= a.nx; ++c) {
+  for (int c = 1; c <= slots && c <= a.nx; ++c) {
     if (forced > 0 && c != forced) continue;
     const int len = (a.nx + c - 1) / c;
+    if (c > 64 && len < 4) break;
     const long long items = (long long)a.n_tiles * ((a.nx + len - 1) / len);
     const long long waves = (items + slots - 1) / slots;
     const double eff = double(items) / (double(waves) * slots) * double(len) / double(len + 2);

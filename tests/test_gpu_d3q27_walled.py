@@ -63,3 +63,26 @@ def test_all_stored_cells(storage, shape, regime, flags, diagnostics):
     if diagnostics:
         assert int(health) == 0
         assert abs(float(mass) - want[0][fluid].sum()) <= 320 * eps * fluid.sum()
+
+
+@pytest.mark.parametrize("storage,shape", [("float32", (700, 16, 32)), ("float32", (300, 3, 4)), ("float64", (515, 9, 33))])
+def test_a_long_column_in_many_chunks(storage, shape):
+    """A domain of one or two tiles is cut into as many chunks along x as there are blocks: the bits of
+    one chunk."""
+    from openhomelbm_b200 import _lib
+    from openhomelbm_b200.lbm3d import LBM_Solver3D
+
+    out = []
+    for chunks in (0, 1):
+        s = LBM_Solver3D(*shape, storage=storage, use_graph=False, with_flag=False)
+        f = s.flows[0]
+        f.moments[0].copy_(torch.tensor(_state(shape, "clamped", 8)))
+        f.moments[1].fill_(7)
+        _lib.set_tuning("d3q27_chunks", chunks)
+        try:
+            _lib.check(_lib.lib().hl_d3q27_stream_collide(f.world_struct(0), 0.02, None, _lib.stream_ptr()), "step")
+        finally:
+            _lib.set_tuning("d3q27_chunks", 0)
+        out.append(f.moments[1].clone())
+    assert torch.equal(*out)
+    assert (out[0][0] != 7).sum() == np.prod([n - 2 for n in shape])

@@ -45,9 +45,9 @@ def measured_peaks():
     return 6650.0, "fallback"
 
 
-# DRAM bytes (read + write) per cell of one stream-collide launch, from one ncu capture of
-# the 256^3 bench workload (profiles/d3q27_sweep_256.md).
-DRAM_BYTES_PER_CELL = {"float32": 1338.7e6 / 256 ** 3, "float16": 663.5e6 / 256 ** 3}
+# DRAM bytes (read + write) per cell of one stream-collide launch, from ncu captures of the 256^3
+# bench workload (profiles/d3q27_sweep_256.md, float16 profiles/d3q27_stream_collide_tma_256_dram.md).
+DRAM_BYTES_PER_CELL = {"float32": 1338.2e6 / 256 ** 3, "float16": 643.2e6 / 256 ** 3}
 
 
 def profile_traffic(n, storage):

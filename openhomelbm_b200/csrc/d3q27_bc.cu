@@ -87,7 +87,14 @@ __device__ __forceinline__ float fma_rn(float a, float b, float c) { return __fm
 __device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
 __device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
-// the equilibrium's stress difference between velocities a and b, one component
+// f_eq_home_3d (envs/lbm3d/lbm_func_3d.py:651-686): S of the unclamped second-order
+// equilibrium populations f_i = w_i (rho - 1 + rho (3 c.u + 4.5 (c.u)^2 - 1.5 u^2)), from
+// deviations f - w (S_aa = (P_aa - (rho-1)/3)/rho, S_ab = P_ab/rho). The D3Q27 weights give
+// sum w c_a c_b = delta_ab / 3, odd moments 0 and sum w c_a c_b c_c c_d = (delta_ab delta_cd +
+// delta_ac delta_bd + delta_ad delta_bc) / 9, so P_ab = (rho - 1) delta_ab / 3 + rho u_a u_b
+// and S_ab = u_a u_b exactly: computed in that closed form, not as the reference's 27-term
+// binary32 sums (which agree with it to their rounding).
+// feq_gap: the difference of that S between velocities a and b, one component.
 template <class S, bool FACE, class R> __device__ __forceinline__ R feq_gap(R a1, R a2, R b1, R b2) {
   if constexpr (S::kEncoded && !FACE) return fma_rn(-b1, b2, mul_rn(a1, a2));
   else return fma_rn(a1, a2, -mul_rn(b1, b2));
@@ -118,14 +125,6 @@ __device__ __forceinline__ void store_cell(const BcArgs& a, long long i, const M
 #pragma unroll
   for (int k = 0; k < 10; ++k) p[k * a.N + i] = S::from_r(raw[k], unsigned(k * a.N + i));
 }
-
-// f_eq_home_3d (envs/lbm3d/lbm_func_3d.py:651-686): S of the unclamped second-order
-// equilibrium populations f_i = w_i (rho - 1 + rho (3 c.u + 4.5 (c.u)^2 - 1.5 u^2)), from
-// deviations f - w (S_aa = (P_aa - (rho-1)/3)/rho, S_ab = P_ab/rho). The D3Q27 weights give
-// sum w c_a c_b = delta_ab / 3, odd moments 0 and sum w c_a c_b c_c c_d = (delta_ab delta_cd +
-// delta_ac delta_bd + delta_ad delta_bc) / 9, so P_ab = (rho - 1) delta_ab / 3 + rho u_a u_b
-// and S_ab = u_a u_b exactly: computed in that closed form, not as the reference's 27-term
-// binary32 sums (which agree with it to their rounding).
 
 // apply_bc_core_3d (envs/lbm3d/lbm_func_3d.py:627-648): new state of boundary cell t from
 // its own old state and its inward neighbour nb.

@@ -19,8 +19,8 @@ struct StepArgs {
   const float* force;
   const int* flag;
   Scale sc;
-  double* partials;        // [gridDim.x] mass partials
-  int* bad_partials;       // [gridDim.x]
+  double* partials;        // [diag_slots] mass partials
+  int* bad_partials;       // [diag_slots]
   int diag_slots;  // partial sums and counts that the diagnostics scratch holds
   unsigned* counter;       // completion counter (returns to 0 after each launch)
   double* mass;

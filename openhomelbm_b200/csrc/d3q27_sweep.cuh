@@ -149,7 +149,7 @@ __device__ __forceinline__ void tensormap_acquire(const CUtensorMap* m) {
   asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;\n" ::"l"(reinterpret_cast<unsigned long long>(m))
                : "memory");
 }
-// Asynchronous copy of one element (4 or 8 bytes); zero-fills when !in.
+// Asynchronous copy of one element; zero-fills when !in.
 template <int BYTES> __device__ __forceinline__ void cp_async_elem(unsigned dst, const void* src, bool in) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;\n" ::"r"(dst), "l"(src), "n"(BYTES), "r"(in ? BYTES : 0)
                : "memory");
@@ -161,7 +161,6 @@ __device__ __forceinline__ void cp_async_arrive(unsigned bar) {
 
 // ---------------------------------------------------------------- lane vectors
 __device__ __forceinline__ P2 vmax_m1(P2 a) { return P2(fmaxf(a.x(), -1.f), fmaxf(a.y(), -1.f)); }
-__device__ __forceinline__ float vmax_m1(float a) { return fmaxf(a, -1.f); }
 __device__ __forceinline__ double vmax_m1(double a) { return ::fmax(a, -1.0); }
 __device__ __forceinline__ P2 reciprocal(P2 x) {
   // the rcp.approx estimate (relative error below 2^-22 by the PTX ISA) and one Newton-Raphson
@@ -180,7 +179,6 @@ __device__ __forceinline__ P2 unless_empty(P2 z, P2 v, float instead) {
 __device__ __forceinline__ double unless_empty(double z, double v, double instead) { return z == -216.0 ? instead : v; }
 __device__ __forceinline__ P2 bcast(P2, float v) { return P2(v, v); }
 __device__ __forceinline__ double bcast(double, double v) { return v; }
-__device__ __forceinline__ float bcast(float, float v) { return v; }
 
 // max(|a|, |b|, |c|), NaN if any is
 __device__ __forceinline__ float max3_abs(float a, float b, float c) {
